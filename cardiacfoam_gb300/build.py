@@ -1,14 +1,17 @@
 """Build libcardiac_gpu.so in-tree for sm_103a (GB300).
 
-Each ionic model is compiled twice from ``csrc/ionic_instance.cu``: the plain
-form with ``--fmad=false`` (FP64 rounding in the host's evaluation order) and
-the mixed form with FMA contraction.  Translation units are compiled in
-parallel; only changed ones are rebuilt.
+Each ionic model is compiled twice from ``csrc/ionic_instance.cu``, the plain
+FP64 form and the mixed form, once per tissue from ``csrc/ionic_tissue.cu`` (the
+plain form with that tissue's constants) and once from ``csrc/ionic_sweep.cu``.
+The FP64 units are compiled with ``--fmad=false``: their multiply-adds are
+written out, so a value rounds alike in every kernel.  Translation units
+are compiled in parallel; only changed ones are rebuilt.
 """
 from __future__ import annotations
 
 import hashlib
 import os
+import re
 import shutil
 import subprocess
 from concurrent.futures import ThreadPoolExecutor
@@ -42,6 +45,12 @@ def nvcc() -> str:
     return cand
 
 
+def tissues(model: str):
+    """Tissue flags of a model, from its generated header."""
+    text = (CSRC / "models" / f"{model}.cuh").read_text()
+    return [int(t) for t in re.search(r"TissueList<([^>]*)>", text).group(1).split(",")]
+
+
 def _units():
     units = []
     # register budget of the ionic kernels: resident 128-thread blocks per SM
@@ -54,12 +63,20 @@ def _units():
         for prec, flags in (("fp64", ["--fmad=false", "-DCFG_FP64=1"]),
                             ("mixed", ["--use_fast_math", "-DCFG_FP64=0"])):
             extra = list(ionic_extra)
+            if prec == "fp64":
+                each = "".join(f"X({t})" for t in tissues(m))
+                extra.append(f"-DCFG_FOR_TISSUES(X)={each}")
             if not unroll and m in STATE_UNROLL:
                 extra.append(f"-DCFG_IONIC_STATE_UNROLL={STATE_UNROLL[m]}")
             if prec == "mixed" and m in MIXED_MIN_BLOCKS:
                 extra.append(f"-DCFG_MIXED_MIN_BLOCKS={MIXED_MIN_BLOCKS[m]}")
             units.append((f"ionic_{m}_{prec}", CSRC / "ionic_instance.cu",
                           flags + [f"-DCFG_MODEL={m}"] + extra))
+        for t in tissues(m):
+            units.append((f"ionic_{m}_tissue{t}", CSRC / "ionic_tissue.cu",
+                          ["--fmad=false", f"-DCFG_MODEL={m}", f"-DCFG_TISSUE={t}"] + ionic_extra))
+        units.append((f"sweep_{m}", CSRC / "ionic_sweep.cu",
+                      ["--fmad=false", f"-DCFG_MODEL={m}"]))
     units.append(("ionic_registry", CSRC / "ionic_registry.cu", []))
     units.append(("ionic", CSRC / "ionic.cu", []))
     units.append(("batch", CSRC / "batch.cu", []))
@@ -114,7 +131,10 @@ def build(force: bool = False, jobs: int | None = None, verbose: bool = False) -
 
     jobs = jobs or max(1, min(len(units), os.cpu_count() or 1))
     with ThreadPoolExecutor(max_workers=jobs) as ex:
-        results = list(ex.map(compile_unit, units))
+        # the longest first: four-warp FP64 kernels of the large models
+        order = sorted(units, key=lambda u: "_tissue" not in u[0] or
+                       not u[0].startswith(("ionic_torord", "ionic_ord")))
+        results = list(ex.map(compile_unit, order))
     rebuilt = any(r for _, r in results)
     if rebuilt or force or not LIB.exists():
         objs = [str(BUILD / f"{n}.o") for n, _, _ in units]

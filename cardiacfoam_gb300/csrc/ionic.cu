@@ -296,7 +296,11 @@ int ionic_autotune(cfg_ionic* ion, double t0, double dt, const double* t_dev, co
     const long long n = ion->n;
     const int nw = ion->ops->n_wide[p], nn = ion->ops->ns - nw;
     const int max_b = ion->ops->max_block[p]();
+    // the plain form's own rule (block 0, threads in blocks of 128) may share a
+    // tile between warps, which no explicit shape does
+    const bool plain = p == CFG_PRECISION_FP64;
     std::vector<int> blocks;
+    if (plain) blocks.push_back(0);
     for (int b = 32; b <= max_b; b *= 2) blocks.push_back(b);
     const int cpts[] = {1, 2, 4};
     double *yw = nullptr, *step = nullptr, *im = nullptr;
@@ -326,6 +330,7 @@ int ionic_autotune(cfg_ionic* ion, double t0, double dt, const double* t_dev, co
     int best_b = saved_b, best_c = saved_c;
     for (int b : blocks)
         for (int c : cpts) {
+            if (b == 0 && c > 1) continue;
             ion->block = b;
             ion->cells_per_thread = c;
             float total = 0.0f;
@@ -366,7 +371,7 @@ int ionic_autotune(cfg_ionic* ion, double t0, double dt, const double* t_dev, co
     cudaStreamSynchronize(s);
     cleanup();
     if (e) return fail(CFG_ERR_CUDA, "autotune failed: %s", cudaGetErrorString(e));
-    if (block_out) *block_out = best_b;
+    if (block_out) *block_out = best_b > 0 ? best_b : max_b;
     if (cpt_out) *cpt_out = best_c;
     if (ms_out) *ms_out = best / float(repeats > 0 ? repeats : 1);
     return CFG_OK;

@@ -23,6 +23,7 @@ namespace cfg {
 // Constants of a uniform tissue with the scale-dependent ones per cell.
 template <class R, class M, int T>
 struct ScaledFold {
+    static constexpr bool kFolded = true;   // divisors are never scaled constants
     const R* dep;   // [NSD] this cell's scale-dependent constants
     CFG_D __forceinline__ R operator()(int i) const
     {
@@ -148,12 +149,9 @@ __global__ void __launch_bounds__(128) batch_fp64_kernel(BatchLaunch p)
         // derivatives a model does not assign stay zero, as in a zeroed dydt
         for (int j = 0; j < 6; ++j)
             for (int i = 0; i < NS; ++i) k6[j][i] = 0.0;
-        CellState<M, double> cs;
+        double y[NS];
 #pragma unroll
-        for (int i = 0; i < NS; ++i) {
-            cs.y[i] = p.yw[(long long)L::slot(i) * p.n + c];
-            cs.yf[i] = cs.y[i];
-        }
+        for (int i = 0; i < NS; ++i) y[i] = p.yw[(long long)L::slot(i) * p.n + c];
         double dep[M::NSD > 0 ? M::NSD : 1];
 #pragma unroll
         for (int j = 0; j < M::NSD; ++j) dep[j] = p.dep[j * p.n + c];
@@ -171,18 +169,18 @@ __global__ void __launch_bounds__(128) batch_fp64_kernel(BatchLaunch p)
             if (dtm < step) step = dtm;
             IonicFailure why;
             const long long nsub =
-                rkf45_solve<M, true, double>(ts, te, cs, step, k6, Kc, T, stim, p.ode, evals, &why);
+                rkf45_solve<M>(ts, te, y, step, k6, Kc, T, stim, p.ode, evals, &why);
             if (nsub < 0) {
                 batch_fail(p, c, why);
                 failed = true;
                 break;
             }
             t = t_new;
-            batch_sample<M>(p, c, k + 1, a, t, cs.y[0],
-                            M::CA_STATE >= 0 ? cs.y[M::CA_STATE] : 0.0);
+            batch_sample<M>(p, c, k + 1, a, t, y[0],
+                            M::CA_STATE >= 0 ? y[M::CA_STATE] : 0.0);
         }
 #pragma unroll
-        for (int i = 0; i < NS; ++i) p.yw[(long long)L::slot(i) * p.n + c] = cs.y[i];
+        for (int i = 0; i < NS; ++i) p.yw[(long long)L::slot(i) * p.n + c] = y[i];
         p.step[c] = step;
         p.t[c] = t;
         if (failed) k = total;

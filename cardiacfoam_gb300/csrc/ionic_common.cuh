@@ -61,6 +61,63 @@ CFG_HD __forceinline__ float cfg_hrcp(float v) { return 1.0f / v; }
 CFG_HD __forceinline__ double cfg_hdiv(double a, double h) { return a / h; }
 CFG_HD __forceinline__ float cfg_hdiv(float a, float h) { return a * h; }
 
+// ---------------------------------------------------------------- plain form
+// GB300 issues one FP64 instruction per SM partition every 64 clocks, so the
+// number of FP64 instructions is the time of the FP64 kernels; the generated
+// <model>_plain.cuh write their right-hand sides with the following.
+
+// a b + c with one rounding, written out: the kernels are compiled without
+// contraction, so every kernel that evaluates an expression rounds it alike
+CFG_HD __forceinline__ double cfg_fma(double a, double b, double c)
+{
+#ifdef __CUDA_ARCH__
+    return __fma_rn(a, b, c);
+#else
+    return std::fma(a, b, c);
+#endif
+}
+
+// a / b by the reciprocal r = RN(1 / b) at hand: the product, corrected once by
+// its exact remainder, which is the correctly rounded quotient but for rare
+// ties (Markstein 1990), in three instructions where the general division
+// takes about nine.  A quotient that is not finite is passed on as it is (the
+// correction would turn an infinity into a NaN).
+CFG_HD __forceinline__ double cfg_quotient(double a, double b, double r)
+{
+    const double q = a * r;
+#ifdef __CUDA_ARCH__
+    if ((__double2hiint(q) & 0x7ff00000) == 0x7ff00000) return q;
+#else
+    if (!std::isfinite(q)) return q;
+#endif
+    return cfg_fma(cfg_fma(-q, b, a), r, q);
+}
+
+// by a constant of the tissue: where the constants KS are known to the
+// compiler (KS::kFolded), so is the reciprocal
+template <class KS>
+CFG_HD __forceinline__ double cfg_cdiv(double a, double c)
+{
+    if constexpr (KS::kFolded) return cfg_quotient(a, c, 1.0 / c);
+    else return a / c;
+}
+
+// A value the tissue form keeps over the PDE step, with its reciprocal where
+// it is a divisor.
+struct CfgSlot {
+    double v, r;
+    CfgSlot() = default;
+    CFG_HD __forceinline__ CfgSlot(double x) : v(x) {}
+    static CFG_HD __forceinline__ CfgSlot divisor(double x)
+    {
+        CfgSlot s(x);
+        s.r = 1.0 / x;
+        return s;
+    }
+    CFG_HD __forceinline__ operator double() const { return v; }
+};
+CFG_HD __forceinline__ double cfg_hdiv(double a, CfgSlot h) { return cfg_quotient(a, h.v, h.r); }
+
 template <int N, class R>
 CFG_HD __forceinline__ R cfg_ipow(R x)
 {

@@ -1,6 +1,5 @@
 // One ionic model in one precision form.  Compiled once per (model,
-// precision) with -DCFG_MODEL=<namespace> -DCFG_FP64=<0|1>; the plain form is
-// built with --fmad=false so FP64 rounding follows the host evaluation order.
+// precision) with -DCFG_MODEL=<namespace> -DCFG_FP64=<0|1>.
 #include <cuda_runtime.h>
 
 #include "ionic_kernels.cuh"
@@ -12,6 +11,11 @@
 #define CFG_CAT3_(a, b, c) a##b##c
 #define CFG_CAT3(a, b, c) CFG_CAT3_(a, b, c)
 #include CFG_STR(models/CFG_MODEL.cuh)
+#if CFG_FP64
+#define CFG_PLAIN_HEADER(m) CFG_STR(models/m##_plain.cuh)
+#define CFG_PLAIN_(m) CFG_PLAIN_HEADER(m)
+#include CFG_PLAIN_(CFG_MODEL)
+#endif
 
 #if CFG_FP64
 #define CFG_PREC_TAG _fp64
@@ -19,34 +23,42 @@
 #define CFG_PREC_TAG _mixed
 #endif
 
+#if CFG_FP64
+using M = cfg::CFG_MODEL::plain::Model;
+#else
 using M = cfg::CFG_MODEL::Model;
+#endif
 static constexpr bool kFP64 = CFG_FP64 != 0;
 
 using cfg::TissueList;
 using Tissues = cfg::CFG_MODEL::TissueSet;
 
-// The plain form runs ionic_step_kernel (one cell per thread, stage arrays
-// per thread); the mixed form runs ionic_mixed_kernel (stage data in shared
-// memory, block size fixed by the model's slice length).
-// `block` threads per block (the plain form: at most 128; the mixed form:
-// at most the model's slice block, 0 = that block) and p.cells_per_thread
-// slots per thread; every slot's arithmetic is independent of both, so the
-// results are too.
+// The plain form runs ionic_step_kernel (one cell per lane, or per four lanes
+// of as many warps); the mixed form runs ionic_mixed_kernel (stage data in
+// shared memory, block size fixed by the model's slice length).
+// `block` threads per block (the plain form: at most 128, 0 = by the rule
+// below; the mixed form: at most the model's slice block, 0 = that block) and
+// p.cells_per_thread slots per thread; every slot's arithmetic is independent
+// of both, so the results are too.
+#if CFG_FP64
+// constants per cell: a warp to a tile of 32 cells
+template <bool SV, int T>
+static void launch_one(const cfg::IonicLaunch& p, cudaStream_t s, int block)
+{
+    static_assert(T == 0, "the kernels of one tissue are in ionic_tissue.cu");
+    cfg::launch_step<M, SV, T>(p, s, block);
+}
+#else
 template <bool SV, int T>
 static void launch_one(const cfg::IonicLaunch& p, cudaStream_t s, int block)
 {
     const long long cpt = p.cells_per_thread > 0 ? p.cells_per_thread : 1;
-    if constexpr (kFP64) {
-        const int b = (block > 0 && block <= 128) ? block : 128;
-        const unsigned grid = unsigned((p.count + b * cpt - 1) / (b * cpt));
-        cfg::ionic_step_kernel<M, true, SV, T><<<grid, b, 0, s>>>(p);
-    } else {
-        using S = cfg::mixed::Slice<M>;
-        const int b = (block > 0 && block <= S::block && block % 32 == 0) ? block : S::block;
-        const unsigned grid = unsigned((p.count + b * cpt - 1) / (b * cpt));
-        cfg::ionic_mixed_kernel<M, SV, T><<<grid, b, size_t(b) * S::len * 4, s>>>(p);
-    }
+    using S = cfg::mixed::Slice<M>;
+    const int b = (block > 0 && block <= S::block && block % 32 == 0) ? block : S::block;
+    const unsigned grid = unsigned((p.count + b * cpt - 1) / (b * cpt));
+    cfg::ionic_mixed_kernel<M, SV, T><<<grid, b, size_t(b) * S::len * 4, s>>>(p);
 }
+#endif
 
 extern "C" int CFG_CAT3(cfg_ionic_max_block_, CFG_MODEL, CFG_PREC_TAG)()
 {
@@ -80,6 +92,24 @@ static cudaError_t prepare_all(TissueList<TS...>)
     return e;
 }
 
+#if CFG_FP64
+// ionic_tissue.cu, compiled once per tissue flag
+#define CFG_CAT5_(a, b, c, d, e) a##b##c##d##e
+#define CFG_CAT5(a, b, c, d, e) CFG_CAT5_(a, b, c, d, e)
+#define CFG_TISSUE_STEP(T) CFG_CAT5(cfg_ionic_step_, CFG_MODEL, _tissue, T, )
+#define CFG_TISSUE_DECL(T) \
+    extern "C" void CFG_TISSUE_STEP(T)(const cfg::IonicLaunch& p, int solve_vm, cudaStream_t s, int block);
+#define CFG_TISSUE_CASE(T) \
+    case T: CFG_TISSUE_STEP(T)(p, solve_vm, s, block); return true;
+CFG_FOR_TISSUES(CFG_TISSUE_DECL)
+static bool launch_uniform(const cfg::IonicLaunch& p, int solve_vm, cudaStream_t s, int block)
+{
+    switch (p.tissue) {
+        CFG_FOR_TISSUES(CFG_TISSUE_CASE)
+    default: return false;
+    }
+}
+#else
 template <int T0, int... TR>
 static bool launch_uniform(const cfg::IonicLaunch& p, cudaStream_t s, int block,
                            TissueList<T0, TR...>)
@@ -91,19 +121,24 @@ static bool launch_uniform(const cfg::IonicLaunch& p, cudaStream_t s, int block,
     if constexpr (sizeof...(TR) > 0) return launch_uniform(p, s, block, TissueList<TR...>{});
     return false;
 }
+#endif
 
 extern "C" cudaError_t CFG_CAT3(cfg_ionic_step_, CFG_MODEL, CFG_PREC_TAG)(
     const cfg::IonicLaunch& p, int solve_vm, cudaStream_t stream, int block)
 {
     if (p.n <= 0 || p.count <= 0) return cudaSuccess;
     const bool uniform = !p.tissue_cell && !p.scales;
-    if (solve_vm) {
-        launch_one<true, 0>(p, stream, block);
-    } else if (uniform && launch_uniform(p, stream, block, Tissues{})) {
-        // tissue-specialised kernel launched
-    } else {
-        launch_one<false, 0>(p, stream, block);
-    }
+    // a uniform tissue without scales runs the kernel that folds its constants;
+    // for the single-cell form only in FP64, whose time is the FP64
+    // instruction count
+#if CFG_FP64
+    if (uniform && launch_uniform(p, solve_vm, stream, block)) return cudaGetLastError();
+#else
+    if (!solve_vm && uniform && launch_uniform(p, stream, block, Tissues{}))
+        return cudaGetLastError();
+#endif
+    if (solve_vm) launch_one<true, 0>(p, stream, block);
+    else launch_one<false, 0>(p, stream, block);
     return cudaGetLastError();
 }
 
@@ -212,51 +247,3 @@ extern "C" cudaError_t CFG_CAT3(cfg_batch_step_, CFG_MODEL, CFG_PREC_TAG)(
     if (p.n <= 0) return cudaSuccess;
     return batch_dispatch(p, tissue, stream, Tissues{});
 }
-
-#if CFG_FP64
-// ---------------------------------------------------------------- sweepCurrent
-// <Model>::sweepCurrent (e.g. TNNP.C:208-272): the states of one cell with
-// state 0 clamped to V = vmin + (vmax - vmin) i / (npts - 1), the first
-// variables function at VOI = 0, one thread per voltage.  Row i of `out` is
-// [states | algebraic | rates] (2 NS + NA doubles).
-// With clamp = 0 the states are taken as they are (one row: the variables
-// of a cell at model time t, as a trace row of ionicModelIO::write holds).
-template <bool SV>
-__global__ void sweep_kernel(const double* y0, const double* C, int tissue, cfg::CfgStimulus stim,
-                             double vmin, double vmax, int npts, double t, int clamp, double* out)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= npts) return;
-    constexpr int NS = M::NS, NA = M::NA;
-    double y[NS];
-    for (int k = 0; k < NS; ++k) y[k] = y0[k];
-    if (clamp) {
-        const double denom = double(npts - 1);
-        y[0] = vmin + (vmax - vmin) * double(i) / denom;
-    }
-    double A[NA > 0 ? NA : 1] = {};
-    double R[NS] = {};
-    const cfg::ConstView<double> K{C};
-    M::template all_variables<double, SV>(t, cfg::ArrayView<double>{y}, K, A, R, tissue, stim);
-    double* row = out + (long long)i * (2 * NS + NA);
-    for (int k = 0; k < NS; ++k) row[k] = y[k];
-    for (int k = 0; k < NA; ++k) row[NS + k] = A[k];
-    for (int k = 0; k < NS; ++k) row[NS + NA + k] = R[k];
-}
-
-extern "C" cudaError_t CFG_CAT3(cfg_ionic_sweep_, CFG_MODEL, )(
-    const double* y0, const double* C, int tissue, int solve_vm, const cfg::CfgStimulus& stim,
-    double vmin, double vmax, int npts, double t, int clamp, double* out, cudaStream_t s)
-{
-    if (npts <= 0) return cudaSuccess;
-    const int block = 64;
-    const unsigned grid = unsigned((npts + block - 1) / block);
-    if (solve_vm)
-        sweep_kernel<true><<<grid, block, 0, s>>>(y0, C, tissue, stim, vmin, vmax, npts, t, clamp,
-                                                  out);
-    else
-        sweep_kernel<false><<<grid, block, 0, s>>>(y0, C, tissue, stim, vmin, vmax, npts, t, clamp,
-                                                   out);
-    return cudaGetLastError();
-}
-#endif
