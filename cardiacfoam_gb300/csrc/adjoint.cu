@@ -227,8 +227,7 @@ struct PcgArgs {
     const double* b;            // [n]
     double* x;                  // [n] in: initial guess; out: solution
     double *r, *z, *p, *ap;     // work
-    double* partial;            // [2 sets][2][blocks]
-    unsigned* bar_count;
+    gsync::Exchange* xch;
     int* bar_abort;
     double tol;                 // ||r||_2 <= tol ||b||_2
     int max_iter;
@@ -236,101 +235,92 @@ struct PcgArgs {
     int* status;                // out: CFG_ERR_PCG when not converged or aborted
 };
 
-__device__ __forceinline__ double amul(const PcgArgs& a, long long c, const double* q)
+__device__ __forceinline__ double amul(const PcgArgs& a, long long c, double d, const double* q)
 {
-    double acc = a.diag[c] * __ldcg(&q[c]);
+    double acc = d * __ldcg(&q[c]);
     const int cnt = a.cnt[c];
     for (int e = 0; e < cnt; ++e) {
         const long long i = (long long)e * a.n + c;
-        acc -= a.coef[i] * __ldcg(&q[a.col[i]]);
+        acc = __fma_rn(-a.coef[i], __ldcg(&q[a.col[i]]), acc);
     }
     return acc;
 }
 
 // Jacobi-preconditioned CG, one cooperative launch, deterministic reductions.
+// An iteration is two passes, each ended by a sum: A z with p = z + beta p and
+// A p = A z + beta A p (linearity), then the update of x, r and z, so only z
+// crosses blocks.  What bounds it is latency (a sheet of 16,384 cells is one
+// row per thread): the two sums and the FP64 operations in a row between them.
+// 91 to 104 us a solve with three barriers per iteration and two more before
+// the first, each an arrival counter followed by a read of the partial sums.
 __global__ void __launch_bounds__(kPcgBlock) k_pcg(PcgArgs a)
 {
     const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long stride = (long long)gridDim.x * blockDim.x;
-    unsigned epoch = 0;
+    unsigned arrivals = 0;
     int set = 0;
-    double s[2] = {0.0, 0.0};
-    // r = b - A x, z = D^-1 r, p = z; sums r.z and b.b
-    for (long long c = first; c < a.n; c += stride) {
-        const double r = a.b[c] - amul(a, c, a.x);
-        const double z = r / a.diag[c];
-        a.r[c] = r;
-        a.z[c] = z;
-        __stcg(&a.p[c], z);
-        s[0] += r * z;
-        s[1] += a.b[c] * a.b[c];
-    }
-    gsync::block_sums<kPcgBlock, 2>(a.partial, set, s);
-    if (!gsync::grid_barrier(a.bar_count, a.bar_abort, epoch)) goto aborted;
-    {
-        double g[2];
-        gsync::grid_sums<2>(a.partial, set, g);
-        set ^= 1;
-        double rz = g[0];
-        const double bnorm = sqrt(g[1]);
-        int it = 0;
-        double rr = 0.0;
-        {
-            // initial residual norm
-            double t[1] = {0.0};
-            for (long long c = first; c < a.n; c += stride) t[0] += a.r[c] * a.r[c];
-            gsync::block_sums<kPcgBlock, 1>(a.partial, set, t);
-            if (!gsync::grid_barrier(a.bar_count, a.bar_abort, epoch)) goto aborted;
-            double gt[1];
-            gsync::grid_sums<1>(a.partial, set, gt);
-            set ^= 1;
-            rr = gt[0];
+    const auto sum = [&](auto& v) {
+        constexpr int K = sizeof(v) / sizeof(v[0]);
+        return gsync::sync_sums<kPcgBlock, K, gsync::SumDouble>(a.xch, a.bar_abort, arrivals, set,
+                                                                gsync::kSpinLimit, v);
+    };
+    int status = 0, it = 0;
+    do {
+        // r = b - A x, z = D^-1 r (published); sums r.z, b.b and r.r
+        double s[3] = {0.0, 0.0, 0.0};
+        for (long long c = first; c < a.n; c += stride) {
+            const double d = a.diag[c], b = a.b[c];
+            const double r = b - amul(a, c, d, a.x);
+            const double z = r / d;
+            a.r[c] = r;
+            __stcg(&a.z[c], z);
+            s[0] += r * z;
+            s[1] += b * b;
+            s[2] += r * r;
         }
-        while (sqrt(rr) > a.tol * bnorm && it < a.max_iter) {
-            // Ap and p.Ap
+        if (!sum(s)) { status = CFG_ERR_PCG; break; }
+        double rz = s[0], rr = s[2], beta = 0.0;
+        // sqrt(rr) <= tol sqrt(b.b), squared
+        const double limit = a.tol * a.tol * s[1];
+        while (rr > limit && it < a.max_iter) {
             double t[1] = {0.0};
             for (long long c = first; c < a.n; c += stride) {
-                const double q = amul(a, c, a.p);
+                double q = amul(a, c, a.diag[c], a.z), p = __ldcg(&a.z[c]);
+                if (it > 0) {
+                    p = __fma_rn(beta, a.p[c], p);
+                    q = __fma_rn(beta, a.ap[c], q);
+                }
+                a.p[c] = p;
                 a.ap[c] = q;
-                t[0] += a.p[c] * q;
+                t[0] += p * q;
             }
-            gsync::block_sums<kPcgBlock, 1>(a.partial, set, t);
-            if (!gsync::grid_barrier(a.bar_count, a.bar_abort, epoch)) goto aborted;
-            double gt[1];
-            gsync::grid_sums<1>(a.partial, set, gt);
-            set ^= 1;
-            const double alpha = rz / gt[0];
-            // x, r, z; r.z and r.r
+            if (!sum(t)) { status = CFG_ERR_PCG; break; }
+            double alpha[1];
+            gsync::block_scalars<1>(it, alpha, [&](int) { return rz / t[0]; });
             double u[2] = {0.0, 0.0};
             for (long long c = first; c < a.n; c += stride) {
-                a.x[c] += alpha * a.p[c];
-                const double r = a.r[c] - alpha * a.ap[c];
+                a.x[c] = __fma_rn(alpha[0], a.p[c], a.x[c]);
+                const double r = __fma_rn(-alpha[0], a.ap[c], a.r[c]);
                 const double z = r / a.diag[c];
                 a.r[c] = r;
-                a.z[c] = z;
+                __stcg(&a.z[c], z);
                 u[0] += r * z;
                 u[1] += r * r;
             }
-            gsync::block_sums<kPcgBlock, 2>(a.partial, set, u);
-            if (!gsync::grid_barrier(a.bar_count, a.bar_abort, epoch)) goto aborted;
-            double gu[2];
-            gsync::grid_sums<2>(a.partial, set, gu);
-            set ^= 1;
-            const double beta = gu[0] / rz;
-            rz = gu[0];
-            rr = gu[1];
+            if (!sum(u)) { status = CFG_ERR_PCG; break; }
+            double next[1];
+            gsync::block_scalars<1>(it + 1, next, [&](int) { return u[0] / rz; });
+            beta = next[0];
+            rz = u[0];
+            rr = u[1];
             ++it;
-            for (long long c = first; c < a.n; c += stride) __stcg(&a.p[c], a.z[c] + beta * a.p[c]);
-            if (!gsync::grid_barrier(a.bar_count, a.bar_abort, epoch)) goto aborted;
         }
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
-            *a.iters = it;
-            if (sqrt(rr) > a.tol * bnorm) atomicOr(a.status, CFG_ERR_PCG);
-        }
-        return;
+        if (rr > limit) status = CFG_ERR_PCG;
+    } while (false);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *a.iters = it;
     }
-aborted:
-    if (threadIdx.x == 0) atomicOr(a.status, CFG_ERR_PCG);
+    if (status && threadIdx.x == 0) atomicOr(a.status, status);
 }
 
 // ------------------------------------------------------------------ elementwise
@@ -476,7 +466,7 @@ struct cfg_adjoint {
     int n_boxes = 0;
     double box_start[8], box_end[8], box_intensity[8];
     double sigma[2] = {0, 0};
-    int pcg_blocks = 0;
+    int pcg_blocks = 0, pcg_block = kPcgBlock;
     bool fp32 = false;          // FP32 right-hand side and its derivative (mixed form)
     cudaStream_t stream = nullptr;
     // device
@@ -489,8 +479,8 @@ struct cfg_adjoint {
     double *d_target = nullptr, *d_trace = nullptr;
     double *d_scales = nullptr, *d_consts = nullptr;
     double *d_y = nullptr, *d_vm = nullptr, *d_vm_old = nullptr, *d_im = nullptr, *d_b = nullptr;
-    double *d_r = nullptr, *d_z = nullptr, *d_p = nullptr, *d_ap = nullptr, *d_partial = nullptr;
-    unsigned* d_bar = nullptr;
+    double *d_r = nullptr, *d_z = nullptr, *d_p = nullptr, *d_ap = nullptr;
+    gsync::Exchange* d_xch = nullptr;
     int *d_abort = nullptr, *d_iters = nullptr, *d_status = nullptr;
     double* d_loss = nullptr;
     // checkpoints and the window
@@ -515,8 +505,8 @@ void adj_free(cfg_adjoint* a)
                     (void*)a->d_probes, (void*)a->d_target, (void*)a->d_trace,
                     (void*)a->d_scales, (void*)a->d_consts, (void*)a->d_y, (void*)a->d_vm,
                     (void*)a->d_vm_old, (void*)a->d_im, (void*)a->d_b, (void*)a->d_r,
-                    (void*)a->d_z, (void*)a->d_p, (void*)a->d_ap, (void*)a->d_partial,
-                    (void*)a->d_bar, (void*)a->d_abort, (void*)a->d_iters, (void*)a->d_status,
+                    (void*)a->d_z, (void*)a->d_p, (void*)a->d_ap, (void*)a->d_xch,
+                    (void*)a->d_abort, (void*)a->d_iters, (void*)a->d_status,
                     (void*)a->d_loss, (void*)a->d_ck_y, (void*)a->d_ck_vm, (void*)a->d_win_y,
                     (void*)a->d_win_vm, (void*)a->d_ybar, (void*)a->d_vbar, (void*)a->d_mu,
                     (void*)a->d_imbar, (void*)a->d_pbar, (void*)a->d_sig_partial})
@@ -539,18 +529,17 @@ int solve(cfg_adjoint* a, const double* b, double* x)
     p.b = b;
     p.x = x;
     p.r = a->d_r; p.z = a->d_z; p.p = a->d_p; p.ap = a->d_ap;
-    p.partial = a->d_partial;
-    p.bar_count = a->d_bar;
+    p.xch = a->d_xch;
     p.bar_abort = a->d_abort;
     p.tol = a->pcg_tol;
     p.max_iter = a->pcg_max_iter;
     p.iters = a->d_iters;
     p.status = a->d_status;
-    CFG_CUDA_TRY(cudaMemsetAsync(a->d_bar, 0, sizeof(unsigned), a->stream));
+    CFG_CUDA_TRY(cudaMemsetAsync(&a->d_xch->count, 0, sizeof(unsigned), a->stream));
     CFG_CUDA_TRY(cudaMemsetAsync(a->d_abort, 0, sizeof(int), a->stream));
     void* args[] = {&p};
     CFG_CUDA_TRY(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(k_pcg), dim3(a->pcg_blocks),
-                                             dim3(kPcgBlock), args, 0, a->stream));
+                                             dim3(a->pcg_block), args, 0, a->stream));
     return CFG_OK;
 }
 
@@ -771,8 +760,11 @@ int cfg_adjoint_create(const cfg_adjoint_desc* d, const cfg_mesh_desc* m, cfg_ad
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pcg, kPcgBlock, 0);
-    const long long want = (n + kPcgBlock - 1) / kPcgBlock;
-    a->pcg_blocks = int(std::min<long long>(want, (long long)sms * std::max(per_sm, 1)));
+    // small sheets in blocks of half the size, on twice the SMs
+    if ((n + kPcgBlock / 2 - 1) / (kPcgBlock / 2) <= sms) a->pcg_block = kPcgBlock / 2;
+    const long long want = (n + a->pcg_block - 1) / a->pcg_block;
+    a->pcg_blocks = int(std::min<long long>(
+        gsync::kMaxBlocks, std::min<long long>(want, (long long)sms * std::max(per_sm, 1))));
     cudaError_t e = cudaSuccess;
     auto alloc = [&](auto** ptr, size_t count) {
         if (!e) e = dmalloc(ptr, count);
@@ -794,8 +786,7 @@ int cfg_adjoint_create(const cfg_adjoint_desc* d, const cfg_mesh_desc* m, cfg_ad
     for (double** v : {&a->d_vm, &a->d_vm_old, &a->d_im, &a->d_b, &a->d_r, &a->d_z, &a->d_p,
                        &a->d_ap, &a->d_vbar, &a->d_mu, &a->d_imbar})
         alloc(v, nn);
-    alloc(&a->d_partial, size_t(4 * std::max(a->pcg_blocks, 1)));
-    alloc(&a->d_bar, 1);
+    alloc(&a->d_xch, 1);
     alloc(&a->d_abort, 1);
     alloc(&a->d_iters, 1);
     alloc(&a->d_status, 1);
@@ -807,6 +798,7 @@ int cfg_adjoint_create(const cfg_adjoint_desc* d, const cfg_mesh_desc* m, cfg_ad
     alloc(&a->d_ybar, size_t(NS) * nn);
     alloc(&a->d_pbar, 6 * nn);
     alloc(&a->d_sig_partial, 2 * size_t(grid_of(n, kBlock)));
+    if (!e) e = cudaMemset(a->d_xch, 0, sizeof(gsync::Exchange));
     if (e) return bail(fail(CFG_ERR_CUDA, "adjoint allocation failed: %s", cudaGetErrorString(e)));
     e = cudaMemcpy(a->d_col, col.data(), slots * sizeof(int), cudaMemcpyHostToDevice);
     if (!e) e = cudaMemcpy(a->d_cnt, cnt.data(), nn, cudaMemcpyHostToDevice);

@@ -31,7 +31,8 @@
 // iteration runs as a kernel sequence with its scalars on the device, two
 // launches per iteration, replayed in chunks from a CUDA graph.  That is the
 // FP64 solve; the mixed form's default is the float-pair, single-reduction
-// solve (k_pcg_pair, one grid barrier per iteration).
+// solve (one grid barrier per iteration): k_pcg_pair_row where every row has a
+// thread, k_pcg_pair with rows in turn beyond.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -465,9 +466,8 @@ constexpr int kCoopBlock = 512;
 struct CoopPcgArgs {
     PcgArgs a;
     double* p_alt;            // second direction buffer
-    double* partial;          // [2 sets][2][gridDim.x]
-    unsigned* bar_count;      // grid barrier (zeroed before the launch)
-    int* bar_abort;
+    cfg::gsync::Exchange* xch;   // its sums, each a grid barrier
+    int* bar_abort;           // a block waited too long (zeroed before the launch)
     long long spin_limit;
 };
 
@@ -521,8 +521,13 @@ __global__ void __launch_bounds__(kCoopBlock, 1) k_pcg_coop(CoopPcgArgs ca)
     const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const double tol = st->tol, rel = st->rel;
     const int max_iter = st->max_iter;
-    unsigned epoch = 0;
+    Exchange* const xch = ca.xch;
+    unsigned arrivals = 0;
     int set = 0;
+    const auto sum = [&](auto& v) {
+        constexpr int K = sizeof(v) / sizeof(v[0]);
+        return sync_sums<kCoopBlock, K, SumDouble>(xch, ca.bar_abort, arrivals, set, ca.spin_limit, v);
+    };
     bool aborted = false;
     double init_res = 0.0, res = 0.0;
     int iter = 0, status = 0;
@@ -540,11 +545,8 @@ __global__ void __launch_bounds__(kCoopBlock, 1) k_pcg_coop(CoopPcgArgs ca)
             s1[0] += a.x[c];
             s1[1] += fabs(rr);
         }
-        block_sums<kCoopBlock, 2>(ca.partial, set, s1);
-        if (!grid_barrier(ca.bar_count, ca.bar_abort, epoch, ca.spin_limit)) { aborted = true; break; }
-        double g1[2];
-        grid_sums<2>(ca.partial, set, g1);
-        set ^= 1;
+        if (!sum(s1)) { aborted = true; break; }
+        const double(&g1)[2] = s1;
         const double avg = g1[0] / double(n);
         // --- normFactor; z = D^-1 r (published), z.r
         double s2[2] = {0.0, 0.0};
@@ -556,11 +558,8 @@ __global__ void __launch_bounds__(kCoopBlock, 1) k_pcg_coop(CoopPcgArgs ca)
             __stcg(&a.z[c], zc);
             s2[1] += zc * rr;
         }
-        block_sums<kCoopBlock, 2>(ca.partial, set, s2);
-        if (!grid_barrier(ca.bar_count, ca.bar_abort, epoch, ca.spin_limit)) { aborted = true; break; }
-        double g2[2];
-        grid_sums<2>(ca.partial, set, g2);
-        set ^= 1;
+        if (!sum(s2)) { aborted = true; break; }
+        const double(&g2)[2] = s2;
         const double normf = g2[0] + 1e-20;
         init_res = g1[1] / normf;
         res = init_res;
@@ -582,16 +581,12 @@ __global__ void __launch_bounds__(kCoopBlock, 1) k_pcg_coop(CoopPcgArgs ca)
                 a.ap[c] = acc;
                 s3[0] += acc * pc;
             }
-            block_sums<kCoopBlock, 1>(ca.partial, set, s3);
-            if (!grid_barrier(ca.bar_count, ca.bar_abort, epoch, ca.spin_limit)) { aborted = true; break; }
-            double g3[1];
-            grid_sums<1>(ca.partial, set, g3);
-            set ^= 1;
+            if (!sum(s3)) { aborted = true; break; }
+            const double(&g3)[1] = s3;
             // checkSingularity and alpha, once per block
             double q3[2];
-            block_scalars<2>(q3, [&](double* v) {
-                v[0] = fabs(g3[0]) / normf < 1e-300 ? 1.0 : 0.0;
-                v[1] = wArA / g3[0];
+            block_scalars<2>(0, q3, [&](int k) {
+                return k == 0 ? (fabs(g3[0]) / normf < 1e-300 ? 1.0 : 0.0) : wArA / g3[0];
             });
             if (q3[0] != 0.0) break;
             const double alpha = q3[1];
@@ -606,17 +601,11 @@ __global__ void __launch_bounds__(kCoopBlock, 1) k_pcg_coop(CoopPcgArgs ca)
                 s4[0] += fabs(rr);
                 s4[1] += zc * rr;
             }
-            block_sums<kCoopBlock, 2>(ca.partial, set, s4);
-            if (!grid_barrier(ca.bar_count, ca.bar_abort, epoch, ca.spin_limit)) { aborted = true; break; }
-            double g4[2];
-            grid_sums<2>(ca.partial, set, g4);
-            set ^= 1;
+            if (!sum(s4)) { aborted = true; break; }
+            const double(&g4)[2] = s4;
             // the residual and beta, once per block
             double q4[2];
-            block_scalars<2>(q4, [&](double* v) {
-                v[0] = g4[0] / normf;
-                v[1] = g4[1] / wArA;
-            });
+            block_scalars<2>(1, q4, [&](int k) { return k == 0 ? g4[0] / normf : g4[1] / wArA; });
             res = q4[0];
             ++iter;
             if (conv(res) || iter >= max_iter) {
@@ -701,8 +690,165 @@ struct PairStep {
     }
 };
 
-template <int W, int B = kCoopBlock>
-__global__ void __launch_bounds__(B, 1) k_pcg_pair(CoopPcgArgs ca, PairPcgArgs q)
+// The solve where every row has a thread (one block per SM): a row's matrix
+// entries, its neighbours' preconditioner and its x, p, r, s and w stay in
+// registers for the whole solve, and only r, s and w are published.  What
+// bounds an iteration is latency: the sum over the blocks, the scalars' chain
+// of pair divisions, and the neighbours' values.  So these are loaded as soon
+// as the blocks have met, before the totals are formed, and the reciprocals
+// that beta and (p, A p) need are formed in the iteration before, which leaves
+// one division in the chain.  A step of 427 phiE iterations on 64,000 rows
+// takes 2.58 ms where the strided form below takes 2.86 (both in blocks of
+// 448), one of 326 on 8,000 rows 1.39 against 1.85 (blocks of 128).
+// Tried without gain: the block's own rows exchanged through shared memory.
+template <int W, int B>
+__global__ void __launch_bounds__(B, 1) k_pcg_pair_row(CoopPcgArgs ca, PairPcgArgs q)
+{
+    using namespace cfg::gsync;
+    using fp::P;
+    const PcgArgs& a = ca.a;
+    const BdOp& op = a.op;
+    PcgScalars* st = a.st;
+    const long long n = op.n;
+    const long long own = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const bool live = own < n;
+    const long long c = live ? own : 0;
+    const P zero = fp::make(0.0f), one = fp::make(1.0f);
+    const P tol = fp::split(st->tol), rel = fp::split(st->rel);
+    const bool use_rel = st->rel > 1e-20;
+    const int max_iter = st->max_iter;
+    const int sh = q.shift;
+    const P small = fp::split(1e-20, sh), count = fp::split(double(n));
+    // published, double-buffered: [0] the previous iteration's values
+    P* r_buf[2] = {reinterpret_cast<P*>(a.r), reinterpret_cast<P*>(a.ax)};
+    P* s_buf[2] = {reinterpret_cast<P*>(a.ap), reinterpret_cast<P*>(ca.p_alt)};
+    P* w_buf[2] = {reinterpret_cast<P*>(a.z), q.pw};
+    Exchange* const xch = ca.xch;
+    unsigned arrivals = 0;
+    int set = 0;
+    const auto sum = [&](auto& v, auto met) {
+        constexpr int K = sizeof(v) / sizeof(v[0]);
+        return sync_sums<B, K, SumPair>(xch, ca.bar_abort, arrivals, set, ca.spin_limit, v, met);
+    };
+    int col[W];
+    P coef[W], nrd[W], nr[W], ns[W], nw[W];
+#pragma unroll
+    for (int e = 0; e < W; ++e) {
+        const long long i = (long long)e * n + c;
+        col[e] = op.col[i];
+        coef[e] = q.pcoef[i];
+        nrd[e] = fp::split(a.rdiag[col[e]], -sh);
+    }
+    const P d = fp::split(a.diag[c], sh), rd = fp::split(a.rdiag[c], -sh);
+    P x = fp::split(a.x[c]);
+    bool aborted = false;
+    P init_res = zero, res = zero;
+    int iter = 0, status = 0;
+    do {
+        // --- A x, r = b - A x; sums of x and |r|
+        const auto row = [&](P dq, auto f) {
+            fp::Acc acc;
+            acc.add_prod(d, dq);
+#pragma unroll
+            for (int e = 0; e < W; ++e) acc.sub_prod(coef[e], f(e));
+            return acc.value();
+        };
+        const P b = fp::split(a.b[c], sh);
+        const P ax = row(x, [&](int e) { return fp::split(a.x[col[e]]); });
+        P r = fp::sub(b, ax);
+        P s1[2] = {live ? x : zero, live ? fp::abs(r) : zero};
+        if (!sum(s1, Nothing())) { aborted = true; break; }
+        // --- normFactor; u = M r (published in w's second buffer)
+        const P pa = fp::mul(row(one, [&](int) { return one; }), fp::div(s1[0], count));
+        const P u = fp::mul(rd, r);
+        if (live) __stcg(&w_buf[1][c], u);
+        P s2[2] = {live ? fp::add(fp::abs(fp::sub(ax, pa)), fp::abs(fp::sub(b, pa))) : zero,
+                   live ? fp::mul(u, r) : zero};
+        if (!sum(s2, Nothing())) { aborted = true; break; }
+        const P normf = fp::add(s2[0], small), inv_normf = fp::div(one, normf);
+        init_res = fp::div(s1[1], normf);
+        const P rel_init = fp::mul(rel, init_res);
+        const auto conv = [&](P rr) {
+            return fp::less(rr, tol) || (use_rel && fp::less(rr, rel_init));
+        };
+        res = init_res;
+        if (conv(res)) break;
+        // --- w = A u; (w, u)
+        P w = row(u, [&](int e) { return __ldcg(&w_buf[1][col[e]]); });
+        if (live) {
+            __stcg(&r_buf[0][c], r);
+            __stcg(&w_buf[0][c], w);
+        }
+        P s3[1] = {live ? fp::mul(w, u) : zero};
+        // the values of an iteration: where they are written, and next time
+        P *rc = r_buf[0], *sc = s_buf[0], *wc = w_buf[0];
+        P *rn = r_buf[1], *sn = s_buf[1], *wn = w_buf[1];
+        // the neighbours' r, s and w of the previous iteration
+        const auto gather = [&] {
+#pragma unroll
+            for (int e = 0; e < W; ++e) {
+                nr[e] = __ldcg(&rc[col[e]]);
+                ns[e] = __ldcg(&sc[col[e]]);
+                nw[e] = __ldcg(&wc[col[e]]);
+            }
+        };
+        if (!sum(s3, gather)) { aborted = true; break; }
+        P gamma = s2[1], delta = s3[0], s = zero, p = zero;
+        P inv_gamma_old = zero, inv_alpha_old = zero;
+        for (;;) {
+            // (p, A p) = delta - beta gamma / alpha_old
+            PairStep ps;
+            ps.first = iter == 0;
+            ps.beta = fp::mul(gamma, inv_gamma_old);
+            const P pap = fp::sub(delta, fp::mul(fp::mul(ps.beta, gamma), inv_alpha_old));
+            if (pap.x == 0.0f) break;   // checkSingularity
+            ps.alpha = fp::div(gamma, pap);
+            ps.nalpha = fp::neg(ps.alpha);
+            inv_gamma_old = fp::div(one, gamma);
+            inv_alpha_old = fp::mul(pap, inv_gamma_old);
+            s = ps.s_next(w, s);
+            const P u_old = fp::mul(rd, r);
+            p = ps.first ? u_old : fp::madd(ps.beta, p, u_old);
+            x = fp::madd(ps.alpha, p, x);
+            r = ps.r_next(r, s);
+            const P un = fp::mul(rd, r);
+            w = row(un, [&](int e) {
+                return fp::mul(nrd[e], ps.r_next(nr[e], ps.s_next(nw[e], ns[e])));
+            });
+            P* t;
+            t = rc, rc = rn, rn = t;
+            t = sc, sc = sn, sn = t;
+            t = wc, wc = wn, wn = t;
+            if (live) {
+                __stcg(&rc[c], r);
+                __stcg(&sc[c], s);
+                __stcg(&wc[c], w);
+            }
+            P s4[3] = {live ? fp::mul(un, r) : zero, live ? fp::mul(w, un) : zero,
+                       live ? fp::abs(r) : zero};
+            if (!sum(s4, gather)) { aborted = true; break; }
+            res = fp::mul(s4[2], inv_normf);
+            ++iter;
+            if (conv(res) || iter >= max_iter) {
+                if (!conv(res)) status = 1;
+                break;
+            }
+            gamma = s4[0];
+            delta = s4[1];
+        }
+    } while (false);
+    if (live && !aborted) a.x[c] = fp::join(x);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        st->iter = iter;
+        st->init_res = fp::join(init_res);
+        st->res = fp::join(res);
+        st->status = aborted ? 2 : status;
+        st->done = 1;
+    }
+}
+
+template <int W>
+__global__ void __launch_bounds__(kCoopBlock, 1) k_pcg_pair(CoopPcgArgs ca, PairPcgArgs q)
 {
     using namespace cfg::gsync;
     using fp::P;
@@ -727,9 +873,13 @@ __global__ void __launch_bounds__(B, 1) k_pcg_pair(CoopPcgArgs ca, PairPcgArgs q
     P* w_new = q.pw;
     P* p = reinterpret_cast<P*>(a.p);
     P* ax = reinterpret_cast<P*>(a.ax);
-    float2* partial = reinterpret_cast<float2*>(ca.partial);
-    unsigned epoch = 0;
+    Exchange* const xch = ca.xch;
+    unsigned arrivals = 0;
     int set = 0;
+    const auto sum = [&](auto& v) {
+        constexpr int K = sizeof(v) / sizeof(v[0]);
+        return sync_sums<kCoopBlock, K, SumPair>(xch, ca.bar_abort, arrivals, set, ca.spin_limit, v);
+    };
     bool aborted = false, started = false;
     P init_res = fp::make(0.0f), res = fp::make(0.0f);
     int iter = 0, status = 0;
@@ -755,11 +905,8 @@ __global__ void __launch_bounds__(B, 1) k_pcg_pair(CoopPcgArgs ca, PairPcgArgs q
             s1[1] = fp::add(s1[1], fp::abs(rc));
         }
         started = true;
-        block_sums_pair<B, 2, 3>(partial, set, s1);
-        if (!grid_barrier(ca.bar_count, ca.bar_abort, epoch, ca.spin_limit)) { aborted = true; break; }
-        P g1[2];
-        grid_sums_pair<2, 3>(partial, set, g1);
-        set ^= 1;
+        if (!sum(s1)) { aborted = true; break; }
+        const P(&g1)[2] = s1;
         const P avg = fp::div(g1[0], count);
         // --- normFactor; u = M r (published in w[1] until w = A u is formed)
         P s2[2] = {fp::make(0.0f), fp::make(0.0f)};
@@ -776,11 +923,8 @@ __global__ void __launch_bounds__(B, 1) k_pcg_pair(CoopPcgArgs ca, PairPcgArgs q
             __stcg(&w_new[c], uc);
             s2[1] = fp::madd(uc, rc, s2[1]);
         }
-        block_sums_pair<B, 2, 3>(partial, set, s2);
-        if (!grid_barrier(ca.bar_count, ca.bar_abort, epoch, ca.spin_limit)) { aborted = true; break; }
-        P g2[2];
-        grid_sums_pair<2, 3>(partial, set, g2);
-        set ^= 1;
+        if (!sum(s2)) { aborted = true; break; }
+        const P(&g2)[2] = s2;
         const P normf = fp::add(g2[0], small);
         init_res = fp::div(g1[1], normf);
         const P rel_init = fp::mul(rel, init_res);
@@ -801,11 +945,8 @@ __global__ void __launch_bounds__(B, 1) k_pcg_pair(CoopPcgArgs ca, PairPcgArgs q
             w_cur[c] = wc;
             s3[0] = fp::madd(wc, __ldcg(&u0[c]), s3[0]);
         }
-        block_sums_pair<B, 1, 3>(partial, set, s3);
-        if (!grid_barrier(ca.bar_count, ca.bar_abort, epoch, ca.spin_limit)) { aborted = true; break; }
-        P g3[1];
-        grid_sums_pair<1, 3>(partial, set, g3);
-        set ^= 1;
+        if (!sum(s3)) { aborted = true; break; }
+        const P(&g3)[1] = s3;
         P gamma = g2[1], delta = g3[0], gamma_old = fp::make(0.0f), alpha_old = fp::make(1.0f);
         for (;;) {
             // the scalars of this iteration; (p, A p) = delta - beta gamma / alpha_old
@@ -850,11 +991,8 @@ __global__ void __launch_bounds__(B, 1) k_pcg_pair(CoopPcgArgs ca, PairPcgArgs q
             }
             // the three sums in one set of three slots; sets alternate, so a
             // set is written again only after every block has read it
-            block_sums_pair<B, 3, 3>(partial, set, s4);
-            if (!grid_barrier(ca.bar_count, ca.bar_abort, epoch, ca.spin_limit)) { aborted = true; break; }
-            P g4[3];
-            grid_sums_pair<3, 3>(partial, set, g4);
-            set ^= 1;
+            if (!sum(s4)) { aborted = true; break; }
+            const P(&g4)[3] = s4;
             res = fp::div(g4[2], normf);
             ++iter;
             P* t = r_cur; r_cur = r_new; r_new = t;
@@ -939,8 +1077,8 @@ struct cfg_bidomain {
     unsigned* d_ticket = nullptr;
     // the persistent solve: grid (0: not available), second direction buffer,
     // its reduction partials and grid barrier
-    int coop_blocks = 0;
-    double *d_p_alt = nullptr, *d_coop_partial = nullptr;
+    int coop_blocks = 0, coop_block = 512;
+    double *d_p_alt = nullptr;
     // float-pair PCG of the persistent solve (CFG_PCG_FLOAT_PAIRS, the mixed
     // form's default): per system [0] phiE, [1] Vm the scaled coefficients
     // and their scale, the iterate and the scaled diagonal as pairs; the
@@ -953,7 +1091,7 @@ struct cfg_bidomain {
     float2 *d_px = nullptr, *d_pdiag = nullptr, *d_prdiag = nullptr, *d_pw = nullptr;
     double max_vol = 0.0, max_row_i = 0.0, max_row_e = 0.0;
     double step_dt = 0.0;
-    unsigned* d_bar = nullptr;
+    cfg::gsync::Exchange* d_xch = nullptr;
     int* d_abort = nullptr;
     long long spin_limit = cfg::gsync::kSpinLimit;
     // kChunk PCG iterations of each system captured as a graph: [0] phiE, [1] Vm
@@ -1012,16 +1150,20 @@ PcgArgs pcg_args(cfg_bidomain* bd, const double* coef, double* x)
 }
 
 // The float-pair solve's kernel for an ELL width and block size
-const void* pair_kernel(int width, int block)
+// row: every row has a thread
+const void* pair_kernel(int width, int block, bool row)
 {
-    if (block == 448)
-        return width == 6 ? (const void*)k_pcg_pair<6, 448>
-             : width == 4 ? (const void*)k_pcg_pair<4, 448> : (const void*)k_pcg_pair<0, 448>;
-    if (block == 384)
-        return width == 6 ? (const void*)k_pcg_pair<6, 384>
-             : width == 4 ? (const void*)k_pcg_pair<4, 384> : (const void*)k_pcg_pair<0, 384>;
-    return width == 6 ? (const void*)k_pcg_pair<6> : width == 4 ? (const void*)k_pcg_pair<4>
-                                                                : (const void*)k_pcg_pair<0>;
+    if (row && width == 6)
+        return block <= 384   ? (const void*)k_pcg_pair_row<6, 384>
+               : block == 448 ? (const void*)k_pcg_pair_row<6, 448>
+                              : (const void*)k_pcg_pair_row<6, 512>;
+    if (row && width == 4)
+        return block <= 384   ? (const void*)k_pcg_pair_row<4, 384>
+               : block == 448 ? (const void*)k_pcg_pair_row<4, 448>
+                              : (const void*)k_pcg_pair_row<4, 512>;
+    return width == 6   ? (const void*)k_pcg_pair<6>
+           : width == 4 ? (const void*)k_pcg_pair<4>
+                        : (const void*)k_pcg_pair<0>;
 }
 
 // kind 0: phiE (coef_e, phiE), 1: Vm (coef_i, Vm)
@@ -1040,10 +1182,9 @@ int pcg_solve(cfg_bidomain* bd, int kind, double tol, double rel, int max_iter,
         *bd->h_st = init;
         CFG_CUDA_TRY(cudaMemcpyAsync(bd->d_st, bd->h_st, sizeof(PcgScalars),
                                      cudaMemcpyHostToDevice, s));
-        CFG_CUDA_TRY(cudaMemsetAsync(bd->d_bar, 0, sizeof(unsigned), s));
+        CFG_CUDA_TRY(cudaMemsetAsync(&bd->d_xch->count, 0, sizeof(unsigned), s));
         CFG_CUDA_TRY(cudaMemsetAsync(bd->d_abort, 0, sizeof(int), s));
-        CoopPcgArgs ca{a, bd->d_p_alt, bd->d_coop_partial, bd->d_bar, bd->d_abort,
-                       bd->spin_limit};
+        CoopPcgArgs ca{a, bd->d_p_alt, bd->d_xch, bd->d_abort, bd->spin_limit};
         if (bd->pair) {
             // the largest diagonal is at most 2 x the largest row sum of the
             // phiE system (setReference doubles one), chi Cm 2 V / dt + the
@@ -1062,8 +1203,9 @@ int pcg_solve(cfg_bidomain* bd, int kind, double tol, double rel, int max_iter,
             }
             PairPcgArgs pa{bd->d_pcoef[kind], shift, bd->d_px, bd->d_pdiag, bd->d_prdiag,
                            bd->d_pw};
+            const bool row = (long long)bd->pair_blocks * bd->pair_block >= bd->n;
             void* params[] = {&ca, &pa};
-            CFG_CUDA_TRY(cudaLaunchCooperativeKernel(pair_kernel(bd->op.width, bd->pair_block),
+            CFG_CUDA_TRY(cudaLaunchCooperativeKernel(pair_kernel(bd->op.width, bd->pair_block, row),
                                                      dim3(bd->pair_blocks), dim3(bd->pair_block),
                                                      params, 0, s));
         } else {
@@ -1071,7 +1213,7 @@ int pcg_solve(cfg_bidomain* bd, int kind, double tol, double rel, int max_iter,
             const void* fn = bd->op.width == 6 ? (const void*)k_pcg_coop<6>
                            : bd->op.width == 4 ? (const void*)k_pcg_coop<4>
                                                : (const void*)k_pcg_coop<0>;
-            CFG_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(bd->coop_blocks), dim3(kCoopBlock),
+            CFG_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(bd->coop_blocks), dim3(bd->coop_block),
                                                      params, 0, s));
         }
         CFG_CUDA_TRY(cudaMemcpyAsync(bd->h_st, bd->d_st, sizeof(PcgScalars),
@@ -1161,10 +1303,10 @@ extern "C" int cfg_bidomain_destroy(cfg_bidomain* bd)
                        &bd->d_grad, &bd->d_dv, &bd->d_diag, &bd->d_rdiag, &bd->d_b, &bd->d_r,
                        &bd->d_z,
                        &bd->d_p, &bd->d_ap, &bd->d_ax, &bd->d_partial, &bd->d_p_alt,
-                       &bd->d_coop_partial, &bd->d_ki, &bd->d_ke, &bd->d_bki, &bd->d_bke,
+                       &bd->d_ki, &bd->d_ke, &bd->d_bki, &bd->d_bke,
                        &bd->d_cv})
         dfree(*p);
-    dfree(bd->d_bar);
+    dfree(bd->d_xch);
     dfree(bd->d_abort);
     dfree(bd->d_pcoef[0]);
     dfree(bd->d_pcoef[1]);
@@ -1403,19 +1545,30 @@ extern "C" int cfg_bidomain_create(const cfg_bidomain_desc* d, const cfg_mesh_de
                     per_sm = std::min(per_sm, k);
             }
             const long long want = (n + kCoopBlock - 1) / kCoopBlock;
-            const long long cap = (long long)sms * per_sm;
+            const long long cap =
+                std::min<long long>((long long)sms * per_sm, cfg::gsync::kMaxBlocks);
             bd->coop_blocks = int(want < cap ? want : cap);
-            // the float-pair solve: the smallest block of 384, 448 or 512
-            // threads whose grid, one row per thread, fits one block per SM,
-            // so that every SM takes part in a small system
+            bd->coop_block = kCoopBlock;
+            // the smallest block whose grid, one row per thread, fits one
+            // block per SM, so that every SM takes part in a small system
+            for (int b : {128, 256, 384})
+                if ((n + b - 1) / b <= sms) {
+                    bd->coop_block = b;
+                    bd->coop_blocks = int((n + b - 1) / b);
+                    break;
+                }
+            // pairs: the same with a register form that stays in registers up
+            // to blocks of 512 (at 8,000 rows 1393 us a step in blocks of
+            // 128, 1804 in 512; at 64,000 2582 in 448, 2724 in 512); beyond
+            // that rows take turns
             bd->pair_block = 512;
-            bd->pair_blocks = bd->coop_blocks;
-            for (int b : {384, 448}) {
+            bd->pair_blocks = int(want < cap ? want : cap);
+            for (int b : {128, 256, 384, 448, 512}) {
                 const long long nb = (n + b - 1) / b;
                 int k = 0;
                 if (nb <= sms &&
                     cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                        &k, pair_kernel(width, b), b, 0) == cudaSuccess && k >= 1) {
+                        &k, pair_kernel(width, b, true), b, 0) == cudaSuccess && k >= 1) {
                     bd->pair_block = b;
                     bd->pair_blocks = int(nb);
                     break;
@@ -1428,9 +1581,8 @@ extern "C" int cfg_bidomain_create(const cfg_bidomain_desc* d, const cfg_mesh_de
         e = dmalloc(&bd->d_p_alt, size_t(n));
         if (!e) e = cudaMemset(bd->d_p_alt, 0, size_t(n) * sizeof(double));
         // two sets of up to three sums per block
-        if (!e) e = dmalloc(&bd->d_coop_partial,
-                            6 * size_t(std::max(bd->coop_blocks, bd->pair_blocks)));
-        if (!e) e = dmalloc(&bd->d_bar, 1);
+        if (!e) e = dmalloc(&bd->d_xch, 1);
+        if (!e) e = cudaMemset(bd->d_xch, 0, sizeof(cfg::gsync::Exchange));
         if (!e) e = dmalloc(&bd->d_abort, 1);
     }
     if (e) return bail(fail(CFG_ERR_CUDA, "bidomain allocation: %s", cudaGetErrorString(e)));

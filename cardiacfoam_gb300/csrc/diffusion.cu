@@ -4,6 +4,7 @@
 // reciprocal are precomputed per dt, so the per-step kernels carry no FP64
 // division (GB300's FP64 pipe, not HBM, would otherwise bound them).
 #include "diffusion_kernels.cuh"
+#include "grid_sync.cuh"
 
 namespace cfg {
 
@@ -28,8 +29,8 @@ __global__ void k_step_begin(DiffusionArgs a)
         st->n_solves = 0;
         st->iter = 0;
         st->step_iters = 0;
-        st->bar_count = 0;
         st->bar_abort = 0;
+        if (a.xch) a.xch->count = 0;
     }
 }
 

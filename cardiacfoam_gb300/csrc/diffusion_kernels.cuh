@@ -23,6 +23,8 @@
 
 namespace cfg {
 
+namespace gsync { struct Exchange; }
+
 constexpr int kDiffBlock = 256;
 constexpr int kMaxSolves = 16;
 
@@ -45,8 +47,8 @@ struct PcgState {
     double sum_x, avg, sum_absr, normf, init_res, res, wArA, wArAold, wApA, alpha, beta;
     double t, t0;         // runTime value and step start
     unsigned int arrive[4];
-    // grid barrier of the persistent diffusion kernel (reset every step)
-    unsigned int bar_count;
+    // a block of the persistent diffusion kernel waited too long (reset every
+    // step)
     int bar_abort;
     // --- statistics of the last step
     int iters[kMaxSolves];
@@ -100,6 +102,7 @@ struct DiffusionArgs {
     // PCG work
     double *b, *r, *z, *ax, *pA, *pB, *ap;
     double* partial;           // [4][nblocks]
+    gsync::Exchange* xch;      // sums of the persistent kernels
     int nblocks;
     PcgState* st;
     // graph control: conditional handles of the PIMPLE and PCG while-nodes

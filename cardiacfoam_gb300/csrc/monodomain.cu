@@ -43,7 +43,7 @@ static void md_free(cfg_monodomain* md)
     dfree(md->d_iion); dfree(md->d_act); dfree(md->d_act_flag); dfree(md->d_box);
     dfree(md->d_diag2); dfree(md->d_rdiag2); dfree(md->d_sumA2); dfree(md->d_b); dfree(md->d_r);
     dfree(md->d_z); dfree(md->d_ax); dfree(md->d_pA); dfree(md->d_pB); dfree(md->d_ap);
-    dfree(md->d_partial); dfree(md->d_st);
+    dfree(md->d_partial); dfree(md->d_xch); dfree(md->d_st);
     for (void** p : {&md->d_nc_gw, &md->d_nc_k, &md->d_nc_om, &md->d_nc_bk, &md->d_grad}) {
         if (*p) cudaFree(*p);
         *p = nullptr;
@@ -314,6 +314,7 @@ static void fill_args(cfg_monodomain* md, double dt)
     a.b = md->d_b; a.r = md->d_r; a.z = md->d_z; a.ax = md->d_ax; a.pA = md->d_pA;
     a.pB = md->d_pB; a.ap = md->d_ap;
     a.partial = md->d_partial;
+    a.xch = md->d_xch;
     a.nblocks = int((md->n + kDiffBlock - 1) / kDiffBlock);
     a.st = md->d_st;
     a.dt = dt;
@@ -413,6 +414,8 @@ int monodomain_create(const cfg_monodomain_desc* d, const cfg_mesh_desc* m, cfg_
     if (!e) e = dmalloc(&md->d_sumA2, 2 * n);
     const int nblocks = int((n + kDiffBlock - 1) / kDiffBlock);
     if (!e) e = dmalloc(&md->d_partial, size_t(4) * nblocks);
+    if (!e) e = dmalloc(&md->d_xch, 1);
+    if (!e) e = cudaMemset(md->d_xch, 0, sizeof(gsync::Exchange));
     if (!e) e = dmalloc(&md->d_act_flag, n);
     if (!e) e = dmalloc(&md->d_st, 1);
     for (size_t c = 0; c < n; ++c) md->max_vol = std::max(md->max_vol, m->volumes[c]);
@@ -521,7 +524,7 @@ int enqueue_step(cfg_monodomain* md, double dt, bool host_control)
         return CFG_OK;
     }
     if (md->persistent) {
-        CFG_CUDA_TRY(launch_implicit_coop(a, md->coop_blocks, s));
+        CFG_CUDA_TRY(launch_implicit_coop(a, s));
         launches += 1;
         if (md->timing) CFG_CUDA_TRY(cudaEventRecord(md->ev[2], s));
         return CFG_OK;

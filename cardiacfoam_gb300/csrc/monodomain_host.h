@@ -48,6 +48,7 @@ struct cfg_monodomain {
     double *d_b = nullptr, *d_r = nullptr, *d_z = nullptr, *d_ax = nullptr, *d_pA = nullptr,
            *d_pB = nullptr, *d_ap = nullptr;
     double* d_partial = nullptr;
+    cfg::gsync::Exchange* d_xch = nullptr;
     // float-pair PCG of the persistent solve (CFG_PCG_FLOAT_PAIRS, the mixed
     // form's default): the scaled operator as pairs and the published
     // iterate; the scale follows from the largest diagonal, bounded by
@@ -109,7 +110,7 @@ int check_step(cfg_monodomain* md);
 int build_step_graph(cfg_monodomain* md, double dt);
 void fill_args_public(cfg_monodomain* md, double dt);
 int coop_grid_blocks(long long n);
-cudaError_t launch_implicit_coop(const DiffusionArgs& a, int blocks, cudaStream_t s);
+cudaError_t launch_implicit_coop(const DiffusionArgs& a, cudaStream_t s);
 // coupling of a conduction network (csrc/purkinje.cu)
 int monodomain_attach_network(cfg_monodomain* md, cfg_purkinje* pk, double* src_total);
 int monodomain_source_total(cfg_monodomain* md, double t0, const int* dep_off,

@@ -102,7 +102,7 @@ static int build_persistent_graph(cfg_monodomain* md, double dt)
         le = ionic_enqueue(md->ion, L);
     }
     if (!le && md->timing) le = cudaEventRecordWithFlags(md->ev[1], s, cudaEventRecordExternal);
-    if (!le) le = launch_implicit_coop(a, md->coop_blocks, s);
+    if (!le) le = launch_implicit_coop(a, s);
     if (!le && md->timing) le = cudaEventRecordWithFlags(md->ev[2], s, cudaEventRecordExternal);
     const cudaError_t ce = cudaStreamEndCapture(s, &g);
     if (le || ce) {
