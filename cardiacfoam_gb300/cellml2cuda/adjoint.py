@@ -28,13 +28,26 @@ adds to ybar[NS] the product of the transposed Jacobian of (dydt, Iion_cm) with
 respect to the states with (dbar, ibar), and to pbar[NSCALE] the same with
 respect to the scalable conductances (SCALE_ORDER: GNa, GCaL, GKr, GKs, GK1,
 Gto), whose values K(C_x) are the already scaled constants.
+
+V is the same at every stage of a PDE step in tissue mode (hoist.py), so the
+mixed form takes the body apart at what depends on V and constants alone:
+
+    adj_hoist<R>(y_V, K, tissue, H)
+    adj_rhs<R>(t, y, K, tissue, H, dydt)                    returns Iion_cm
+    adj_rhs_vjp<R>(t, y, K, tissue, H, dbar, ibar, ybar, pbar, hbar)
+    adj_hoist_vjp<R>(y_V, K, tissue, hbar)                  returns dV
+
+adj_rhs_vjp adds the adjoint of the values H to hbar; the derivative being
+linear in it, one adj_hoist_vjp of the sum over all stages replaces the part of
+every stage's rhs_vjp that runs through them.
 """
 from __future__ import annotations
 
 from typing import Dict, List, Tuple
 
-from .cexpr import Bin, Call, Cond, Node, Num, Ref, Unary, Var
+from .cexpr import Bin, Call, Cond, Node, Num, Ref, Unary, Var, walk
 from .emit import SCALABLE, SCALE_ORDER, _int_exponent, _is_half, ident
+from .hoist import analyse
 from .model import Assign, Fatal, If, Model, use_before_def
 
 _CMP = ("==", "!=", "<", ">", "<=", ">=", "&&", "||")
@@ -82,6 +95,8 @@ class _Gen:
         self.value: Dict[int, str] = {}     # id(node) -> value name
         self.alg_bar: Dict[str, str] = {}   # algebraic value name -> its adjoint accumulator
         self.states_read = set()
+        self.varying: Dict[str, bool] = {}  # H slots that depend on V
+        self.alg_ref: Dict[int, str] = {}
 
     def tmp(self, prefix="t") -> str:
         self.n += 1
@@ -101,6 +116,8 @@ class _Gen:
                 return f"p_{e.name}" if e.name in self.params else f"K(C_{e.name})"
             if e.array == "ALGEBRAIC":
                 return self.defined.get(e.name, "R(0)")
+            if e.array == "H":
+                return f"H[{e.name}]"
             raise ValueError(f"read of {e.array} in the right-hand side")
         if isinstance(e, Var):
             if e.name == "tissueFlag":
@@ -220,6 +237,9 @@ class _Gen:
                 out.append(f"{ind}ybar[S_{e.name}] += {g};")
             elif e.array == "CONSTANTS" and e.name in self.params:
                 out.append(f"{ind}pbar[SCALE_{self.params[e.name]}] += {g};")
+            elif e.array == "H":
+                if e.name in self.varying:
+                    out.append(f"{ind}hbar[{e.name}] += {g};")
             elif e.array == "ALGEBRAIC" and id(e) in self.alg_ref:
                 out.append(f"{ind}{self.alg_ref[id(e)]} += {g};")
             return
@@ -306,17 +326,12 @@ class _Gen:
         self.acc(e, t, out, ind)
 
 
-def emit_rhs_vjp(m: Model) -> str:
-    body = tissue_mode_body(m.rates)
-    early = use_before_def(m.rates)
-    gen = _Gen(m, early)
-    gen.alg_ref = {}
-    fwd: List[str] = []
+def _walk_body(gen: _Gen, body, fwd: List[str]):
+    """Forward code of the statements; their (statement, adjoint name) pairs.
+    Assignments to H (a value kept per cell) have H as target array."""
     targets: List[Tuple[Assign, str]] = []
     for st in body:
         t = st.target
-        if t.array == "RATES" and t.name == m.states[0]:
-            continue                                  # the PDE owns Vm
         # record, for the reverse sweep, which value each algebraic read refers to
         for r in _alg_reads(st.expr):
             if r.name in gen.defined:
@@ -327,23 +342,47 @@ def emit_rhs_vjp(m: Model) -> str:
             fwd.append(f"    {name} = {v};")
             gen.defined[t.name] = name
             gen.decl.append(f"    R b{name} = R(0);")
-            targets.append((st, name))
+            targets.append((st, f"b{name}"))
         elif t.array == "RATES":
             targets.append((st, f"dbar[S_{t.name}]"))
+        elif t.array == "H":
+            targets.append((st, f"hbar[{t.name}]"))
         else:
             raise ValueError(f"assignment to {t.array} in the right-hand side")
-    iion = gen.defined.get(m.iion_name)
-    if iion is None:
-        raise ValueError(f"{m.name}: the right-hand side does not compute {m.iion_name}")
-    rev: List[str] = [f"    b{iion} += ibar;"]
+    return targets
+
+
+def _reverse(gen: _Gen, targets) -> List[str]:
+    rev: List[str] = []
     for st, name in reversed(targets):
-        g = name if name.startswith("dbar") else f"b{name}"
         if name.startswith("dbar"):
-            rev.append(f"    {{ const R g0 = {g};")
+            rev.append(f"    {{ const R g0 = {name};")
             gen.push(st.expr, "g0", rev, "      ")
             rev.append("    }")
         else:
-            gen.push(st.expr, g, rev, "    ")
+            gen.push(st.expr, name, rev, "    ")
+    return rev
+
+
+def _states_and_params(gen: _Gen) -> List[str]:
+    return [f"    const R y_{s} = y[S_{s}];" for s in gen.m.states if s in gen.states_read] + \
+           [f"    const R p_{c} = K(C_{c});" for c in gen.params]
+
+
+def _without_v_rate(m: Model) -> List[Assign]:
+    """The body without RATES of V: the PDE owns Vm."""
+    return [st for st in tissue_mode_body(m.rates)
+            if not (st.target.array == "RATES" and st.target.name == m.states[0])]
+
+
+def emit_rhs_vjp(m: Model) -> str:
+    gen = _Gen(m, use_before_def(m.rates))
+    fwd: List[str] = []
+    targets = _walk_body(gen, _without_v_rate(m), fwd)
+    iion = gen.defined.get(m.iion_name)
+    if iion is None:
+        raise ValueError(f"{m.name}: the right-hand side does not compute {m.iion_name}")
+    rev: List[str] = [f"    b{iion} += ibar;"] + _reverse(gen, targets)
     L: List[str] = []
     L.append("// Reverse-mode derivative of rhs<R, false> (tissue mode): adds to ybar the")
     L.append("// transposed Jacobian of (dydt without V, Iion_cm) with respect to the states")
@@ -353,11 +392,7 @@ def emit_rhs_vjp(m: Model) -> str:
              "const R* dbar, R ibar, R* ybar, R* pbar)")
     L.append("{")
     L.append("    (void)t; (void)tissue;")
-    for s in m.states:
-        if s in gen.states_read:
-            L.append(f"    const R y_{s} = y[S_{s}];")
-    for c, key in gen.params.items():
-        L.append(f"    const R p_{c} = K(C_{c});")
+    L.extend(_states_and_params(gen))
     L.extend(gen.decl)
     L.extend(fwd)
     L.extend(rev)
@@ -365,8 +400,133 @@ def emit_rhs_vjp(m: Model) -> str:
     return "\n".join(L) + "\n"
 
 
+def take_apart(m: Model):
+    """The body without RATES of V as (statements of H, the other statements with
+    H in them, H slot -> whether it depends on V).  H holds the algebraics of V
+    and constants that the others read, and the largest subexpressions of the
+    others that read V and constants (no scalable one) alone and hold a special
+    function."""
+    body = _without_v_rate(m)
+    h = analyse(m, m.rates)
+    inv = set(h.invariant)
+    slots: Dict[Node, str] = {}
+    varying: Dict[str, bool] = {}
+    defined: set = set()
+
+    def reads_v(e: Node) -> bool:
+        return any(isinstance(n, Ref) and n.array in ("STATES", "ALGEBRAIC") for n in walk(e))
+
+    def whole(e: Node) -> bool:
+        special = False
+        for n in walk(e):
+            if isinstance(n, Var) and n.name not in ("tissueFlag", "dimension"):
+                return False
+            if isinstance(n, Call):
+                if n.fn == "computeIstim":
+                    return False
+                special |= n.fn in ("exp", "log", "sqrt", "tanh", "tissueSelect") or (
+                    n.fn == "pow" and _int_exponent(n.args[1]) is None)
+            if isinstance(n, Ref) and (
+                    (n.array == "STATES" and n.name != m.states[0]) or n.array == "RATES" or
+                    (n.array == "CONSTANTS" and n.name in SCALABLE[m.name].values()) or
+                    (n.array == "ALGEBRAIC" and n.name not in inv & defined)):
+                return False
+        return special
+
+    def slot(e: Node) -> Ref:
+        if e not in slots:
+            slots[e] = str(len(slots))
+            varying[slots[e]] = reads_v(e)
+        return Ref("H", slots[e])
+
+    def rewrite(e: Node) -> Node:
+        if isinstance(e, (Num, Var)):
+            return e
+        if isinstance(e, Ref):
+            if e.array == "ALGEBRAIC" and e.name in inv and e.name in defined:
+                return slot(e)
+            return Ref(e.array, e.name)
+        if whole(e):
+            return slot(e)
+        if isinstance(e, Unary):
+            return Unary(e.op, rewrite(e.e))
+        if isinstance(e, Bin):
+            return Bin(e.op, rewrite(e.l), rewrite(e.r))
+        if isinstance(e, Cond):
+            return Cond(rewrite(e.c), rewrite(e.a), rewrite(e.b))
+        return Call(e.fn, tuple(rewrite(x) for x in e.args))
+
+    first, rest = [], []
+    for st in body:
+        if st.target.array == "ALGEBRAIC" and st.target.name in inv:
+            first.append(st)
+            defined.add(st.target.name)
+        else:
+            rest.append(Assign(st.target, rewrite(st.expr), st.line))
+    first += [Assign(Ref("H", k), e, 0) for e, k in slots.items()]
+    return first, rest, varying
+
+
+def emit_split(m: Model) -> str:
+    first, rest, varying = take_apart(m)
+    vm = m.states[0]
+    L = [f"constexpr int ADJ_NH = {len(varying)};",
+         "// What the right-hand side has of V and constants alone (the same at every",
+         "// stage of a PDE step).",
+         "template <class R, class KS>",
+         f"__device__ __forceinline__ void adj_hoist(R y_{vm}, const KS& K, int tissue, R* H)",
+         "{",
+         "    (void)tissue;"]
+    gen = _Gen(m, [])
+    fwd: List[str] = []
+    targets = _walk_body(gen, first, fwd)
+    L += gen.decl + fwd
+    L += [f"    H[{st.target.name}] = {gen.value.get(id(st.expr)) or gen.leaf(st.expr)};"
+          for st, _ in targets if st.target.array == "H"]
+    L += ["}", "",
+          "// Their derivative: the adjoint of V for the adjoint hbar of H.",
+          "template <class R, class KS>",
+          f"__device__ __forceinline__ R adj_hoist_vjp(R y_{vm}, const KS& K, int tissue, "
+          "const R* hbar)",
+          "{",
+          "    (void)tissue;",
+          f"    R ybar[1] = {{R(0)}};"]
+    gen = _Gen(m, [])
+    fwd = []
+    targets = _walk_body(gen, first, fwd)
+    targets = [(st, n) for st, n in targets
+               if not (st.target.array == "H" and not varying[st.target.name])]
+    rev = [x.replace(f"ybar[S_{vm}]", "ybar[0]") for x in _reverse(gen, targets)]
+    L += gen.decl + fwd + rev + ["    return ybar[0];", "}", ""]
+
+    gen = _Gen(m, use_before_def(m.rates))
+    gen.varying = {k for k, v in varying.items() if v}
+    fwd = []
+    targets = _walk_body(gen, rest, fwd)
+    iion = gen.defined[m.iion_name]
+    L += ["// The right-hand side with them; returns Iion_cm.",
+          "template <class R, class KS>",
+          "__device__ __forceinline__ R adj_rhs(double t, const R* y, const KS& K, int tissue, "
+          "const R* H, R* dydt)",
+          "{",
+          "    (void)t; (void)tissue;"]
+    decl = [d for d in gen.decl if not d.startswith("    R ba")]
+    L += _states_and_params(gen) + decl + fwd
+    L += [f"    dydt[S_{st.target.name}] = {gen.value.get(id(st.expr)) or gen.leaf(st.expr)};"
+          for st, _ in targets if st.target.array == "RATES"]
+    L += [f"    return {iion};", "}", "",
+          "// Its derivative: as rhs_vjp, and to hbar the adjoint of H.",
+          "template <class R, class KS>",
+          "__device__ __forceinline__ void adj_rhs_vjp(double t, const R* y, const KS& K, "
+          "int tissue, const R* H, const R* dbar, R ibar, R* ybar, R* pbar, R* hbar)",
+          "{",
+          "    (void)t; (void)tissue;"]
+    rev = [f"    b{iion} += ibar;"] + _reverse(gen, targets)
+    L += _states_and_params(gen) + gen.decl + fwd + rev + ["}"]
+    return "\n".join(L) + "\n"
+
+
 def _alg_reads(e: Node):
-    from .cexpr import walk
     for n in walk(e):
         if isinstance(n, Ref) and n.array == "ALGEBRAIC":
             yield n
@@ -384,5 +544,6 @@ def emit_adjoint_header(m: Model, src_rel: str) -> str:
          f"namespace cfg {{ namespace {ns} {{",
          ""]
     L.append(emit_rhs_vjp(m))
+    L.append(emit_split(m))
     L.append(f"}} }}  // namespace cfg::{ns}")
     return "\n".join(L) + "\n"

@@ -1,6 +1,7 @@
 // Differentiable monodomain steps and their adjoint: FP64, or with the
-// ionic right-hand side and its derivative in FP32 (mixed form; states,
-// adjoint accumulations, PCG and the conductivity derivative stay FP64).
+// ionic right-hand side and its derivative in FP32 (mixed form; its sums over
+// stages are float pairs; states, adjoints, PCG and the conductivity derivative
+// stay FP64).
 //
 // Forward step n -> n+1 on an orthogonal mesh (implicit Euler ddt, one
 // linear solve per step):
@@ -30,6 +31,7 @@
 #include <cstring>
 #include <vector>
 
+#include "float_pair.cuh"
 #include "grid_sync.cuh"
 #include "host_common.h"
 #include "ionic_kernels.cuh"
@@ -53,12 +55,11 @@ constexpr double vm_map_slope()
                                       : MAP == CFG_VM_IDENTITY ? 1.0 : 1000.0;
 }
 
-// constants of cell c from the [NC][n] table, read as R
-template <class R>
+// constants of cell c from the [NC][n] table
 struct ColView {
     const double* c;
     long long n, cell;
-    CFG_D __forceinline__ R operator()(int i) const { return R(c[(long long)i * n + cell]); }
+    CFG_D __forceinline__ double operator()(int i) const { return c[(long long)i * n + cell]; }
 };
 
 struct IonicArgs {
@@ -94,126 +95,359 @@ __device__ __forceinline__ Tableau tableau()
                    {0.0, c2, c3, c4, c5, c6}};
 }
 
-// The six stages of one RKF45 substep from the (double) state y: stage
-// inputs Y_s = y + h sum_j a_sj k_j accumulated in double and handed to the
-// right-hand side in R; k_s = f(Y_s) in R.
-template <class R>
+// ------------------------------------------------------------------ FP64
+// The six stages of one RKF45 substep from the state y: stage inputs
+// Y_s = y + h sum_j a_sj k_j; k_s = f(Y_s).
 __device__ __forceinline__ void stages(double t, double h, const double* y,
-                                       const ColView<R>& K, int tissue, R (*k)[NS],
-                                       R (*Y)[NS])
+                                       const ColView& K, int tissue, double (*k)[NS],
+                                       double (*Y)[NS])
 {
     const Tableau T = tableau();
     const CfgStimulus none{};
     for (int s = 0; s < 6; ++s) {
         for (int i = 0; i < NS; ++i) {
             double acc = 0.0;
-            for (int j = 0; j < s; ++j) acc += T.a[s][j] * double(k[j][i]);
-            Y[s][i] = R(y[i] + h * acc);
-            k[s][i] = R(0);           // RATES of V stay zero in tissue mode
+            for (int j = 0; j < s; ++j) acc += T.a[s][j] * k[j][i];
+            Y[s][i] = y[i] + h * acc;
+            k[s][i] = 0.0;            // RATES of V stay zero in tissue mode
         }
-        M::rates<R, false>(t + T.c[s] * h, ArrayView<R>{Y[s]}, K, k[s], tissue, none);
+        M::rates<double, false>(t + T.c[s] * h, ArrayView<double>{Y[s]}, K, k[s], tissue, none);
     }
 }
 
-// y += h sum_s b_s k_s, in double
-template <class R>
-__device__ __forceinline__ void substep(double h, double* y, const R (*k)[NS])
+// y += h sum_s b_s k_s
+__device__ __forceinline__ void substep(double h, double* y, const double (*k)[NS])
 {
     const Tableau T = tableau();
     for (int i = 0; i < NS; ++i) {
         double acc = 0.0;
-        for (int s = 0; s < 6; ++s) acc += T.b[s] * double(k[s][i]);
+        for (int s = 0; s < 6; ++s) acc += T.b[s] * k[s][i];
         y[i] += h * acc;
     }
 }
 
-// Forward ionic update of one PDE step with fixed substeps.  R = double is
-// the FP64 form; R = float evaluates the right-hand side in FP32 and keeps
-// the states and their accumulation in FP64.
-template <class R>
+// Forward ionic update of one PDE step with fixed substeps.
 __global__ void __launch_bounds__(kBlock) k_ionic_forward(IonicArgs a)
 {
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= a.n) return;
-    const ColView<R> K{a.consts, a.n, c};
+    const ColView K{a.consts, a.n, c};
     double y[NS];
     for (int i = 0; i < NS; ++i) y[i] = a.y[(long long)i * a.n + c];
     y[0] = vm_to_state0<M::VM_MAP>(a.vm[c]);
-    R k[6][NS], Y[6][NS];
+    double k[6][NS], Y[6][NS];
     const double h = a.dtm / a.substeps;
     for (int j = 0; j < a.substeps; ++j) {
-        stages<R>(a.t0 + j * h, h, y, K, a.tissue, k, Y);
-        substep<R>(h, y, k);
+        stages(a.t0 + j * h, h, y, K, a.tissue, k, Y);
+        substep(h, y, k);
     }
-    R yr[NS], d[NS];
-    for (int i = 0; i < NS; ++i) {
-        yr[i] = R(y[i]);
-        d[i] = R(0);
-    }
+    double d[NS] = {};
     const CfgStimulus none{};
-    const R iion = M::rates<R, false>(a.t0 + a.dtm, ArrayView<R>{yr}, K, d, a.tissue, none);
-    a.im[c] = double(iion) * M::IION_SCALE;
+    const double iion =
+        M::rates<double, false>(a.t0 + a.dtm, ArrayView<double>{y}, K, d, a.tissue, none);
+    a.im[c] = iion * M::IION_SCALE;
     for (int i = 0; i < NS; ++i) a.y[(long long)i * a.n + c] = y[i];
 }
 
 // Reverse of one PDE step of the ionic update (the same arithmetic as the
-// forward recomputed, then the stages backwards through rhs_vjp<R>); the
-// adjoints accumulate in double.
-template <class R>
+// forward recomputed, then the stages backwards through rhs_vjp).
 __global__ void __launch_bounds__(kBlock) k_ionic_reverse(IonicArgs a)
 {
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= a.n) return;
     const Tableau T = tableau();
-    const ColView<R> K{a.consts, a.n, c};
+    const ColView K{a.consts, a.n, c};
     const double h = a.dtm / a.substeps;
     // forward again, keeping the start of every substep
     double ys[kMaxSub + 1][NS];
     for (int i = 0; i < NS; ++i) ys[0][i] = a.y_start[(long long)i * a.n + c];
     ys[0][0] = vm_to_state0<M::VM_MAP>(a.vm[c]);
-    R k[6][NS], Y[6][NS];
+    double k[6][NS], Y[6][NS];
     for (int j = 0; j < a.substeps; ++j) {
         for (int i = 0; i < NS; ++i) ys[j + 1][i] = ys[j][i];
-        stages<R>(a.t0 + j * h, h, ys[j], K, a.tissue, k, Y);
-        substep<R>(h, ys[j + 1], k);
+        stages(a.t0 + j * h, h, ys[j], K, a.tissue, k, Y);
+        substep(h, ys[j + 1], k);
     }
     double pb[6] = {0, 0, 0, 0, 0, 0};
     double yb[NS];
     for (int i = 0; i < NS; ++i) yb[i] = a.ybar[(long long)i * a.n + c];
     yb[0] = 0.0;                      // the next step overwrites state 0 with Vm
-    R Yb[NS], dbR[NS], pbR[6], yr[NS];
-    auto vjp = [&](double t, const R* y, const R* dbar, R ibar) {
-        for (int i = 0; i < NS; ++i) Yb[i] = R(0);
-        for (int q = 0; q < 6; ++q) pbR[q] = R(0);
-        tnnp::rhs_vjp<R>(t, y, K, a.tissue, dbar, ibar, Yb, pbR);
-        for (int q = 0; q < 6; ++q) pb[q] += double(pbR[q]);
+    double Yb[NS], db[NS], pq[6];
+    auto vjp = [&](double t, const double* y, const double* dbar, double ibar) {
+        for (int i = 0; i < NS; ++i) Yb[i] = 0.0;
+        for (int q = 0; q < 6; ++q) pq[q] = 0.0;
+        tnnp::rhs_vjp<double>(t, y, K, a.tissue, dbar, ibar, Yb, pq);
+        for (int q = 0; q < 6; ++q) pb[q] += pq[q];
     };
     // the current at the end of the step
-    for (int i = 0; i < NS; ++i) {
-        yr[i] = R(ys[a.substeps][i]);
-        dbR[i] = R(0);
-    }
-    vjp(a.t0 + a.dtm, yr, dbR, R(a.imbar[c] * M::IION_SCALE));
-    for (int i = 0; i < NS; ++i) yb[i] += double(Yb[i]);
+    for (int i = 0; i < NS; ++i) db[i] = 0.0;
+    vjp(a.t0 + a.dtm, ys[a.substeps], db, a.imbar[c] * M::IION_SCALE);
+    for (int i = 0; i < NS; ++i) yb[i] += Yb[i];
     double kb[6][NS];
     for (int j = a.substeps - 1; j >= 0; --j) {
-        stages<R>(a.t0 + j * h, h, ys[j], K, a.tissue, k, Y);
+        stages(a.t0 + j * h, h, ys[j], K, a.tissue, k, Y);
         for (int s = 0; s < 6; ++s)
             for (int i = 0; i < NS; ++i) kb[s][i] = h * T.b[s] * yb[i];
         // yb stays as the adjoint of the substep's start (identity part)
         for (int s = 5; s >= 0; --s) {
-            for (int i = 0; i < NS; ++i) dbR[i] = R(kb[s][i]);
-            dbR[0] = R(0);                // RATES of V are not part of the map
-            vjp(a.t0 + j * h + T.c[s] * h, Y[s], dbR, R(0));
-            for (int i = 0; i < NS; ++i) yb[i] += double(Yb[i]);
+            for (int i = 0; i < NS; ++i) db[i] = kb[s][i];
+            db[0] = 0.0;                  // RATES of V are not part of the map
+            vjp(a.t0 + j * h + T.c[s] * h, Y[s], db, 0.0);
+            for (int i = 0; i < NS; ++i) yb[i] += Yb[i];
             for (int l = 0; l < s; ++l)
-                for (int i = 0; i < NS; ++i) kb[l][i] += h * T.a[s][l] * double(Yb[i]);
+                for (int i = 0; i < NS; ++i) kb[l][i] += h * T.a[s][l] * Yb[i];
         }
     }
     a.vbar[c] += yb[0] * vm_map_slope<M::VM_MAP>();
     yb[0] = 0.0;
     for (int i = 0; i < NS; ++i) a.ybar[(long long)i * a.n + c] = yb[i];
     for (int q = 0; q < 6; ++q) a.pbar[(long long)q * a.n + c] += pb[q];
+}
+
+// ------------------------------------------------------------------ mixed
+// The right-hand side and its derivative in FP32.  The stage sums, and the sums
+// of the adjoints over stages, are float pairs (48 bits, exact products) that
+// are rounded to FP32 only as inputs of the right-hand side; states and
+// adjoints are FP64 in memory and get the step's change added in FP64.
+//
+// What bounds these kernels is the instructions of a warp: 16,384 cells are one
+// warp for each of 512 of the chip's 608 SM partitions.  The FP64 sums they
+// replace (some 50 operations and conversions a state and substep, 64 clocks
+// each) were most of a step.  V is the same at every stage, so what depends on
+// it alone is evaluated once a step (adj_hoist) and differentiated once
+// (adj_hoist_vjp of the stages' summed adjoints).  The reverse keeps the stage
+// inputs of its forward pass in a workspace instead of forming them twice.
+//
+// The constants that depend on no conductance scale are launch arguments, the
+// scaled ones the cell's, in registers.  (Folding the former at compile time is
+// 4 % faster, but it rounds what is derived from them otherwise.)
+constexpr int kMixedBlock = 64;
+
+struct CellConsts {
+    const float* tissue;        // [NC]
+    float sd[tnnp::NSD];
+    __device__ __forceinline__ CellConsts(const float* t, const float* c, long long n,
+                                          long long cell)
+        : tissue(t)
+    {
+#pragma unroll
+        for (int k = 0; k < tnnp::NSD; ++k) sd[k] = c[k * n + cell];
+    }
+    __device__ __forceinline__ float operator()(int i) const
+    {
+        return tnnp::sd_slot(i) >= 0 ? sd[tnnp::sd_slot(i)] : tissue[i];
+    }
+};
+
+struct PairTableau {
+    fp::P a[7][6];              // h a_sj; row 6: h b_j
+    double c[6];
+};
+
+struct MixedArgs {
+    IonicArgs a;
+    PairTableau T;
+    float tissue[M::NC];        // the tissue's constants
+    const float* consts;        // [NSD][n] scaled constants
+    float* ws;                  // [6 substeps + 1][NS - 1][threads] stage inputs (reverse)
+};
+
+// Adjoints are scaled by 2^kBarShift, so that the pairs' low parts of small ones
+// stay above FP32's smallest number.
+constexpr int kBarShift = 32;
+constexpr double kBarUnit = 1.0 / 4294967296.0;
+
+// One substep of (y, and its change dy since the start of the step); keep(s, Y)
+// is given the stage inputs.  The stages are a loop that is not unrolled, with
+// the rates in shared memory (thread by thread, rows of a block's threads):
+// unrolled, the six right-hand sides are some 6000 instructions, and the one
+// warp of a partition waits for instructions half of the time (80 us for
+// 46 in the forward kernel).
+using Rates = float[6][NS][kMixedBlock];
+
+template <class F>
+__device__ __forceinline__ void mixed_substep(const MixedArgs& g, double t, double h,
+                                              const CellConsts& K, const float* H, Rates& k,
+                                              fp::P (&y)[NS], fp::P (&dy)[NS], F keep)
+{
+    const int tid = threadIdx.x;
+#pragma unroll 1
+    for (int s = 0; s <= 6; ++s) {       // 6: the substep's end
+        fp::Acc d[NS];
+#pragma unroll 1
+        for (int j = 0; j < s; ++j) {
+            const fp::P w = g.T.a[s][j];
+#pragma unroll
+            for (int i = 1; i < NS; ++i) d[i].add_prod(w, k[j][i][tid]);
+        }
+        if (s == 6) {
+#pragma unroll
+            for (int i = 1; i < NS; ++i) {
+                y[i] = fp::add(y[i], d[i].value());
+                dy[i] = fp::add(dy[i], d[i].value());
+            }
+            break;
+        }
+        float Y[NS], ks[NS];
+        Y[0] = y[0].x;
+#pragma unroll
+        for (int i = 1; i < NS; ++i) {
+            const fp::P v = fp::two_sum(y[i].x, d[i].h);
+            Y[i] = __fadd_rn(v.x, __fadd_rn(v.y, __fadd_rn(y[i].y, d[i].l)));
+        }
+        keep(s, Y);
+        tnnp::adj_rhs<float>(t + g.T.c[s] * h, Y, K, g.a.tissue, H, ks);
+#pragma unroll
+        for (int i = 1; i < NS; ++i) k[s][i][tid] = ks[i];
+    }
+}
+
+__device__ __forceinline__ void mixed_start(const double* y0, double vm, long long n, long long c,
+                                            fp::P (&y)[NS], fp::P (&dy)[NS])
+{
+    y[0] = fp::split(vm_to_state0<M::VM_MAP>(vm));
+#pragma unroll
+    for (int i = 1; i < NS; ++i) {
+        y[i] = fp::split(y0[(long long)i * n + c]);
+        dy[i] = fp::make(0.0f);
+    }
+}
+
+// Forward ionic update of one PDE step: 254 us in FP64 sums, 46 us now
+// (16,384 cells, 5 substeps).
+__global__ void __launch_bounds__(kMixedBlock) k_ionic_forward_mixed(
+    const __grid_constant__ MixedArgs g)
+{
+    const IonicArgs& a = g.a;
+    const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= a.n) return;
+    const CellConsts K(g.tissue, g.consts, a.n, c);
+    fp::P y[NS], dy[NS];
+    mixed_start(a.y, a.vm[c], a.n, c, y, dy);
+    float H[tnnp::ADJ_NH];
+    tnnp::adj_hoist<float>(y[0].x, K, g.a.tissue, H);
+    __shared__ Rates k;
+    const double h = a.dtm / a.substeps;
+    for (int j = 0; j < a.substeps; ++j)
+        mixed_substep(g, a.t0 + j * h, h, K, H, k, y, dy, [](int, const float*) {});
+    float yr[NS], d[NS];
+#pragma unroll
+    for (int i = 0; i < NS; ++i) yr[i] = y[i].x;
+    const float iion = tnnp::adj_rhs<float>(a.t0 + a.dtm, yr, K, g.a.tissue, H, d);
+    a.im[c] = double(iion) * M::IION_SCALE;
+    a.y[c] = vm_to_state0<M::VM_MAP>(a.vm[c]);
+#pragma unroll
+    for (int i = 1; i < NS; ++i) a.y[(long long)i * a.n + c] += fp::join(dy[i]);
+}
+
+// Reverse of one PDE step of the ionic update: the forward pass again, keeping
+// the stage inputs, then the current at the end of the step and the stages
+// backwards.  With yb the adjoint of a substep's end and Yb_s that of the stage
+// inputs, the adjoint of rate s is h b_s yb + sum_{l > s} h a_ls Yb_l, and that
+// of the substep's start yb + sum_s Yb_s.  989 us in FP64 sums with the stages
+// formed twice, 119 us now (16,384 cells, 5 substeps).
+__global__ void __launch_bounds__(kMixedBlock) k_ionic_reverse_mixed(
+    const __grid_constant__ MixedArgs g)
+{
+    const IonicArgs& a = g.a;
+    const long long slot = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long slots = (long long)gridDim.x * blockDim.x;
+    const double h = a.dtm / a.substeps;
+    const int last = 6 * a.substeps, tid = threadIdx.x;
+    __shared__ Rates yk;                 // forward: the rates; backward: Yb
+    for (long long c = slot; c < a.n; c += slots) {
+        const CellConsts K(g.tissue, g.consts, a.n, c);
+        float H[tnnp::ADJ_NH], V;
+        {
+            fp::P y[NS], dy[NS];
+            mixed_start(a.y_start, a.vm[c], a.n, c, y, dy);
+            V = y[0].x;
+            tnnp::adj_hoist<float>(V, K, g.a.tissue, H);
+            float* w = g.ws + slot;
+            for (int j = 0; j < a.substeps; ++j)
+                mixed_substep(g, a.t0 + j * h, h, K, H, yk, y, dy, [&](int, const float* Y) {
+#pragma unroll
+                    for (int i = 1; i < NS; ++i, w += slots) *w = Y[i];
+                });
+#pragma unroll
+            for (int i = 1; i < NS; ++i, w += slots) *w = y[i].x;
+        }
+        fp::P yb[NS];
+        fp::Acc dyb[NS], hb[tnnp::ADJ_NH], pb[6];
+#pragma unroll
+        for (int i = 1; i < NS; ++i)
+            yb[i] = fp::split(a.ybar[(long long)i * a.n + c], kBarShift);
+        int s = 0;
+#pragma unroll 1
+        for (int it = last; it >= 0; --it) {
+            float Y[NS], dbar[NS], Ys[NS], hbar[tnnp::ADJ_NH], pbar[6];
+            Y[0] = V;
+            dbar[0] = 0.0f;          // RATES of V are not part of the map
+            Ys[0] = 0.0f;
+            const float* w = g.ws + (long long)it * (NS - 1) * slots + slot;
+#pragma unroll
+            for (int i = 1; i < NS; ++i) {
+                Y[i] = w[(i - 1) * slots];
+                dbar[i] = 0.0f;
+                Ys[i] = 0.0f;
+            }
+#pragma unroll
+            for (int q = 0; q < tnnp::ADJ_NH; ++q) hbar[q] = 0.0f;
+#pragma unroll
+            for (int q = 0; q < 6; ++q) pbar[q] = 0.0f;
+            const bool end = it == last;
+            float ibar = 0.0f;
+            if (end) {
+                ibar = fp::split(a.imbar[c] * M::IION_SCALE, kBarShift).x;
+            } else {
+                fp::Acc d[NS];
+                const fp::P b = g.T.a[6][s];
+#pragma unroll
+                for (int i = 1; i < NS; ++i) d[i].add_prod(b, yb[i]);
+#pragma unroll 1
+                for (int l = s + 1; l < 6; ++l) {
+                    const fp::P w = g.T.a[l][s];
+#pragma unroll
+                    for (int i = 1; i < NS; ++i) d[i].add_prod(w, yk[l][i][tid]);
+                }
+#pragma unroll
+                for (int i = 1; i < NS; ++i) dbar[i] = __fadd_rn(d[i].h, d[i].l);
+            }
+            tnnp::adj_rhs_vjp<float>(0.0, Y, K, g.a.tissue, H, dbar, ibar, Ys, pbar, hbar);
+            dyb[0].add(Ys[0]);
+#pragma unroll
+            for (int q = 0; q < tnnp::ADJ_NH; ++q) hb[q].add(hbar[q]);
+#pragma unroll
+            for (int q = 0; q < 6; ++q) pb[q].add(pbar[q]);
+#pragma unroll
+            for (int i = 1; i < NS; ++i) {
+                dyb[i].add(Ys[i]);
+                yk[s][i][tid] = Ys[i];
+            }
+            if (s == 0) {            // the end of the step, or a substep's start
+                fp::Acc d[NS];
+#pragma unroll 1
+                for (int l = end ? 0 : 5; l >= 0; --l)
+#pragma unroll
+                    for (int i = 1; i < NS; ++i) d[i].add(yk[l][i][tid]);
+#pragma unroll
+                for (int i = 1; i < NS; ++i) yb[i] = fp::add(yb[i], d[i].value());
+            }
+            s = s == 0 ? 5 : s - 1;
+        }
+        float hbar[tnnp::ADJ_NH];
+#pragma unroll
+        for (int q = 0; q < tnnp::ADJ_NH; ++q) hbar[q] = hb[q].value().x;
+        dyb[0].add(tnnp::adj_hoist_vjp<float>(V, K, g.a.tissue, hbar));
+        a.vbar[c] += fp::join(dyb[0].value()) * (kBarUnit * vm_map_slope<M::VM_MAP>());
+        a.ybar[c] = 0.0;
+#pragma unroll
+        for (int i = 1; i < NS; ++i)
+            a.ybar[(long long)i * a.n + c] += fp::join(dyb[i].value()) * kBarUnit;
+#pragma unroll
+        for (int q = 0; q < 6; ++q)
+            a.pbar[(long long)q * a.n + c] += fp::join(pb[q].value()) * kBarUnit;
+    }
 }
 
 // ------------------------------------------------------------------ PCG
@@ -428,7 +662,7 @@ __global__ void k_probes(int np, const int* probes, const double* vm, const doub
 
 // constants per cell: initConsts with the cell's conductance scales
 __global__ void k_consts(long long n, int tissue, const double* scales, double* consts,
-                         double* y)
+                         float* constsf, double* y)
 {
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= n) return;
@@ -438,6 +672,9 @@ __global__ void k_consts(long long n, int tissue, const double* scales, double* 
     for (int q = 0; q < 6; ++q) sc[q] = scales[(long long)q * n + c];
     M::init(C, y0, tissue, sc);
     for (int i = 0; i < M::NC; ++i) consts[(long long)i * n + c] = C[i];
+    if (constsf)
+        for (int k = 0; k < tnnp::NSD; ++k)
+            constsf[(long long)k * n + c] = float(C[tnnp::sd_const(k)]);
     if (y)
         for (int i = 0; i < NS; ++i) y[(long long)i * n + c] = y0[i];
 }
@@ -478,6 +715,8 @@ struct cfg_adjoint {
     int* d_probes = nullptr;
     double *d_target = nullptr, *d_trace = nullptr;
     double *d_scales = nullptr, *d_consts = nullptr;
+    float *d_constsf = nullptr, *d_ws = nullptr;      // mixed form
+    int mixed_blocks = 0;                             // of the reverse
     double *d_y = nullptr, *d_vm = nullptr, *d_vm_old = nullptr, *d_im = nullptr, *d_b = nullptr;
     double *d_r = nullptr, *d_z = nullptr, *d_p = nullptr, *d_ap = nullptr;
     gsync::Exchange* d_xch = nullptr;
@@ -503,7 +742,8 @@ void adj_free(cfg_adjoint* a)
     for (void* p : {(void*)a->d_col, (void*)a->d_cnt, (void*)a->d_gl, (void*)a->d_gt,
                     (void*)a->d_coef, (void*)a->d_diag, (void*)a->d_vol, (void*)a->d_box,
                     (void*)a->d_probes, (void*)a->d_target, (void*)a->d_trace,
-                    (void*)a->d_scales, (void*)a->d_consts, (void*)a->d_y, (void*)a->d_vm,
+                    (void*)a->d_scales, (void*)a->d_consts, (void*)a->d_constsf,
+                    (void*)a->d_ws, (void*)a->d_y, (void*)a->d_vm,
                     (void*)a->d_vm_old, (void*)a->d_im, (void*)a->d_b, (void*)a->d_r,
                     (void*)a->d_z, (void*)a->d_p, (void*)a->d_ap, (void*)a->d_xch,
                     (void*)a->d_abort, (void*)a->d_iters, (void*)a->d_status,
@@ -558,6 +798,33 @@ IonicArgs ionic_args(cfg_adjoint* a, long long step)
     return g;
 }
 
+MixedArgs mixed_args(cfg_adjoint* a, const IonicArgs& g)
+{
+    const double ra[6][5] = {{0, 0, 0, 0, 0},
+                             {rkf::a21, 0, 0, 0, 0},
+                             {rkf::a31, rkf::a32, 0, 0, 0},
+                             {rkf::a41, rkf::a42, rkf::a43, 0, 0},
+                             {rkf::a51, rkf::a52, rkf::a53, rkf::a54, 0},
+                             {rkf::a61, rkf::a62, rkf::a63, rkf::a64, rkf::a65}};
+    const double rb[6] = {rkf::b1, 0.0, rkf::b3, rkf::b4, rkf::b5, rkf::b6};
+    const auto pair = [](double v) { return make_float2(float(v), float(v - double(float(v)))); };
+    const double h = a->dtm / a->substeps;
+    MixedArgs m{};
+    m.a = g;
+    const double rc[6] = {0.0, rkf::c2, rkf::c3, rkf::c4, rkf::c5, rkf::c6};
+    for (int s = 0; s < 6; ++s) {
+        for (int j = 0; j < 5; ++j) m.T.a[s][j] = pair(h * ra[s][j]);
+        m.T.a[6][s] = pair(h * rb[s]);
+        m.T.c[s] = rc[s];
+    }
+    double C[M::NC] = {}, y[NS] = {};
+    M::init(C, y, a->tissue, nullptr);
+    for (int i = 0; i < M::NC; ++i) m.tissue[i] = float(C[i]);
+    m.consts = a->d_constsf;
+    m.ws = a->d_ws;
+    return m;
+}
+
 StepArgs step_args(cfg_adjoint* a, long long step)
 {
     StepArgs s{};
@@ -586,9 +853,10 @@ int forward_step(cfg_adjoint* a, long long step)
     const size_t bytes = sizeof(double) * size_t(a->n);
     CFG_CUDA_TRY(cudaMemcpyAsync(a->d_vm_old, a->d_vm, bytes, cudaMemcpyDeviceToDevice, s));
     if (a->fp32)
-        k_ionic_forward<float><<<grid_of(a->n, kBlock), kBlock, 0, s>>>(ionic_args(a, step));
+        k_ionic_forward_mixed<<<grid_of(a->n, kMixedBlock), kMixedBlock, 0, s>>>(
+            mixed_args(a, ionic_args(a, step)));
     else
-        k_ionic_forward<double><<<grid_of(a->n, kBlock), kBlock, 0, s>>>(ionic_args(a, step));
+        k_ionic_forward<<<grid_of(a->n, kBlock), kBlock, 0, s>>>(ionic_args(a, step));
     k_rhs<<<grid_of(a->n, kBlock), kBlock, 0, s>>>(step_args(a, step));
     CFG_CUDA_TRY(cudaGetLastError());
     return solve(a, a->d_b, a->d_vm);     // the previous Vm is the initial guess
@@ -618,7 +886,8 @@ int set_parameters(cfg_adjoint* a, const double* log_gna, const double* log_gk1,
     cudaStream_t s = a->stream;
     CFG_CUDA_TRY(cudaMemcpyAsync(a->d_scales, sc.data(), sc.size() * sizeof(double),
                                  cudaMemcpyHostToDevice, s));
-    k_consts<<<grid_of(n, kBlock), kBlock, 0, s>>>(n, a->tissue, a->d_scales, a->d_consts, a->d_y);
+    k_consts<<<grid_of(n, kBlock), kBlock, 0, s>>>(n, a->tissue, a->d_scales, a->d_consts,
+                                                   a->d_constsf, a->d_y);
     CFG_CUDA_TRY(cudaGetLastError());
     // A = chi Cm V/dt + L(sigma): coef = sigma_l G_l + sigma_t G_t per ELL slot
     const size_t slots = size_t(a->width) * size_t(n);
@@ -782,6 +1051,19 @@ int cfg_adjoint_create(const cfg_adjoint_desc* d, const cfg_mesh_desc* m, cfg_ad
     alloc(&a->d_trace, size_t(std::max<long long>(a->n_samples * d->n_probes, 1)));
     alloc(&a->d_scales, 6 * nn);
     alloc(&a->d_consts, size_t(M::NC) * nn);
+    if (a->fp32) {
+        // the reverse's threads take cells in turn, so that its stage inputs
+        // need a workspace for the resident threads only
+        int res = 0;
+        if (!e)
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&res, k_ionic_reverse_mixed,
+                                                              kMixedBlock, 0);
+        a->mixed_blocks = int(std::min<long long>((long long)grid_of(n, kMixedBlock),
+                                                  (long long)sms * std::max(res, 1)));
+        alloc(&a->d_constsf, size_t(tnnp::NSD) * nn);
+        alloc(&a->d_ws, size_t(6 * a->substeps + 1) * (NS - 1) * kMixedBlock *
+                            size_t(a->mixed_blocks));
+    }
     alloc(&a->d_y, size_t(NS) * nn);
     for (double** v : {&a->d_vm, &a->d_vm_old, &a->d_im, &a->d_b, &a->d_r, &a->d_z, &a->d_p,
                        &a->d_ap, &a->d_vbar, &a->d_mu, &a->d_imbar})
@@ -919,8 +1201,10 @@ int cfg_adjoint_backward(cfg_adjoint* a, double* grad_log_gna, double* grad_log_
             ia.imbar = a->d_imbar;
             ia.vbar = a->d_vbar;
             ia.pbar = a->d_pbar;
-            if (a->fp32) k_ionic_reverse<float><<<g, kBlock, 0, s>>>(ia);
-            else k_ionic_reverse<double><<<g, kBlock, 0, s>>>(ia);
+            if (a->fp32)
+                k_ionic_reverse_mixed<<<a->mixed_blocks, kMixedBlock, 0, s>>>(mixed_args(a, ia));
+            else
+                k_ionic_reverse<<<g, kBlock, 0, s>>>(ia);
             CFG_CUDA_TRY(cudaGetLastError());
         }
         if (int rc = check(a)) return rc;

@@ -100,6 +100,20 @@ struct Acc {
         h = s.x;
         l = __fadd_rn(l, __fadd_rn(s.y, e));
     }
+    __device__ __forceinline__ void add_prod(P a, float b)
+    {
+        const float p = __fmul_rn(a.x, b);
+        const float e = __fmaf_rn(a.y, b, __fmaf_rn(a.x, b, -p));
+        const P s = two_sum(h, p);
+        h = s.x;
+        l = __fadd_rn(l, __fadd_rn(s.y, e));
+    }
+    __device__ __forceinline__ void add(float b)
+    {
+        const P s = two_sum(h, b);
+        h = s.x;
+        l = __fadd_rn(l, s.y);
+    }
     __device__ __forceinline__ void sub_prod(P a, P b) { add_prod(neg(a), b); }
     __device__ __forceinline__ P value() const { return quick(h, l); }
 };
