@@ -14,10 +14,9 @@
 // into BFS levels, so one block eliminates a whole level at once: every
 // parent of the level subtracts its children's contributions in the order the
 // reference visits them (reverse BFS), then the next level up; substitution
-// runs level by level downwards.  Each accumulator sees the reference's
-// operations in the reference's order, so the solution is bitwise the
-// sequential one.  The matrix coefficients depend only on dt and the graph,
-// and are assembled on the host (in the reference's order) when dt changes.
+// runs level by level downwards.  The matrix depends only on dt and the graph:
+// it is assembled on the host (in the reference's order) and its elimination
+// formed there when dt changes.
 //
 // Coupling: per terminal (PVJ) the tissue cell holding the junction (the
 // nearest cell centre) and the cells whose centres lie within pvjRadius; the
@@ -41,79 +40,133 @@ namespace {
 
 constexpr int kPkBlock = 1024;
 
-// rhs = Vm - dt Iion + dt Iapp / (chi Cm); Iapp from the root stimulus and
-// the terminal currents (assembleAppliedCurrent); diag reset to its base
-struct PkRhsArgs {
-    long long n;
+// Nodes by their position in BFS order: the nodes of a level, and the children of
+// a node, are contiguous.
+struct CableArgs {
+    int n, n_levels;
     double dt, chicm, t0;
     int root;
     double root_start, root_end, root_intensity;
     const int* term_off;    // [n+1] node -> its terminals (in terminal order)
     const int* term_idx;
     const double* term_current;
-    const double* vm;
     const double* iion;
-    const double* diag0;
-    double* diag;
-    double* rhs;
-};
-
-__global__ void k_pk_rhs(PkRhsArgs a)
-{
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.n) return;
-    double app = 0.0;
-    if (i == a.root && a.t0 >= a.root_start && a.t0 <= a.root_end) app += a.root_intensity;
-    for (int k = a.term_off[i]; k < a.term_off[i + 1]; ++k) app -= a.term_current[a.term_idx[k]];
-    a.rhs[i] = a.vm[i] - a.dt * a.iion[i] + a.dt * app / a.chicm;
-    a.diag[i] = a.diag0[i];
-}
-
-struct HinesArgs {
-    int n_levels;
-    const int* level_off;   // [n_levels+1] ranges of `order` (BFS order = by level)
-    const int* order;
-    const int* parent;
-    const int* child_off;   // [n+1] children of each node in reverse BFS order
-    const int* children;
-    const double* pc;       // row child -> column parent
-    const double* cc;       // row parent -> column child
-    double* diag;
-    double* rhs;
     double* vm;
+    const int* level_off;   // [n_levels+1] positions
+    const int* level;       // [n] level of a position
+    const int* order;       // [n] position -> node
+    const int* parent;      // [n] position of the parent
+    const int* child;       // [n+1] first child's position
+    const double* factor;   // [n] row parent -> column child over the eliminated diagonal
+    const double* up;       // [n] row child -> column parent over the eliminated diagonal
+    const double* diag;     // [n] eliminated diagonal
+    double* rhs;            // [n] work, where shared memory does not hold the network
 };
 
-// One block: elimination from the deepest level up, then substitution down.
-__global__ void __launch_bounds__(kPkBlock) k_pk_hines(HinesArgs a)
+// bytes of shared memory of the shared form
+constexpr size_t cable_bytes(size_t n, size_t levels)
 {
-    for (int L = a.n_levels - 1; L >= 1; --L) {
-        // parents on level L-1 take their children's contributions
-        for (int k = a.level_off[L - 1] + threadIdx.x; k < a.level_off[L]; k += blockDim.x) {
-            const int p = a.order[k];
-            double d = a.diag[p], r = a.rhs[p];
-            for (int j = a.child_off[p]; j < a.child_off[p + 1]; ++j) {
-                const int c = a.children[j];
-                const double factor = a.cc[c] / a.diag[c];
-                d -= factor * a.pc[c];
-                r -= factor * a.rhs[c];
-            }
-            a.diag[p] = d;
-            a.rhs[p] = r;
+    return 3 * n * sizeof(double) + (2 * n + 1 + levels + 1) * sizeof(int);
+}
+constexpr size_t kCableShared = 200 * 1024;
+
+// One block: the right-hand side Vm - dt Iion + dt Iapp / (chi Cm), with Iapp from
+// the root stimulus and the terminal currents (assembleAppliedCurrent), its
+// elimination from the deepest level up, and the substitution down.
+//
+// What bounds it is the chain over the levels, twice 37 for a network of 379
+// nodes.  The matrix is that of dt, so its elimination is done when dt is set and
+// a step's chain has neither a division nor a read of global memory (SHARED: up to
+// some 6,000 nodes; larger networks keep theirs in global memory).  A network of
+// at most a block's threads has a thread per node, whose factors and neighbours
+// wait in registers for its level.  Those 379 nodes: 75 us with factors formed on
+// the way, node lists read from global memory and a kernel of its own for the
+// right-hand side; 25.7 us with threads that take a level's nodes in turn,
+// 22 us with a thread per node.
+template <bool SHARED>
+__global__ void __launch_bounds__(kPkBlock) k_pk_cable(const __grid_constant__ CableArgs a)
+{
+    extern __shared__ double cable_mem[];
+    double* x = a.rhs;
+    const double *factor = a.factor, *up = a.up;
+    const int *child = a.child, *parent = a.parent, *off = a.level_off;
+    const bool row = SHARED && a.n <= blockDim.x;   // a thread per node
+    if constexpr (SHARED) x = cable_mem;
+    if (SHARED && !row) {
+        double* f = cable_mem + a.n;
+        double* u = f + a.n;
+        int* c = reinterpret_cast<int*>(u + a.n);
+        int* p = c + a.n + 1;
+        int* l = p + a.n;
+        for (int k = threadIdx.x; k < a.n; k += blockDim.x) {
+            f[k] = a.factor[k];
+            u[k] = a.up[k];
+            c[k] = a.child[k];
+            p[k] = a.parent[k];
         }
-        __syncthreads();
+        if (threadIdx.x == 0) c[a.n] = a.child[a.n];
+        for (int k = threadIdx.x; k <= a.n_levels; k += blockDim.x) l[k] = a.level_off[k];
+        factor = f, up = u, child = c, parent = p, off = l;
     }
-    if (threadIdx.x == 0) {
-        const int root = a.order[0];
-        a.vm[root] = a.rhs[root] / a.diag[root];
+    for (int k = threadIdx.x; k < a.n; k += blockDim.x) {
+        const int i = a.order[k];
+        double app = 0.0;
+        if (i == a.root && a.t0 >= a.root_start && a.t0 <= a.root_end) app += a.root_intensity;
+        for (int q = a.term_off[i]; q < a.term_off[i + 1]; ++q)
+            app -= a.term_current[a.term_idx[q]];
+        x[k] = a.vm[i] - a.dt * a.iion[i] + a.dt * app / a.chicm;
+    }
+    if (row) {
+        const int k = threadIdx.x;
+        const bool live = k < a.n;
+        const int level = live ? a.level[k] : -1;
+        const int c0 = live ? a.child[k] : 0, c1 = live ? a.child[k + 1] : 0;
+        const int p = live ? a.parent[k] : 0;
+        const double f1 = c1 > c0 ? a.factor[c1 - 1] : 0.0;
+        const double f2 = c1 > c0 + 1 ? a.factor[c1 - 2] : 0.0;
+        const double u = live ? a.up[k] : 0.0, d = live ? a.diag[k] : 1.0;
+        double r = live ? x[k] : 0.0;
+        __syncthreads();
+        for (int L = a.n_levels - 2; L >= 0; --L) {
+            if (level == L && c1 > c0) {
+                r -= f1 * x[c1 - 1];
+                if (c1 > c0 + 1) r -= f2 * x[c1 - 2];
+                for (int j = c1 - 3; j >= c0; --j) r -= factor[j] * x[j];
+                x[k] = r;
+            }
+            __syncthreads();
+        }
+        r /= d;
+        if (live) x[k] = r;
+        __syncthreads();
+        for (int L = 1; L < a.n_levels; ++L) {
+            if (level == L) {
+                r -= u * x[p];
+                x[k] = r;
+            }
+            __syncthreads();
+        }
+        if (live) a.vm[a.order[k]] = r;
+        return;
     }
     __syncthreads();
-    for (int L = 1; L < a.n_levels; ++L) {
-        for (int k = a.level_off[L] + threadIdx.x; k < a.level_off[L + 1]; k += blockDim.x) {
-            const int c = a.order[k];
-            a.vm[c] = (a.rhs[c] - a.pc[c] * a.vm[a.parent[c]]) / a.diag[c];
+    for (int L = a.n_levels - 2; L >= 0; --L) {
+        // parents take their children's contributions, the last child first
+        for (int k = off[L] + threadIdx.x; k < off[L + 1]; k += blockDim.x) {
+            double r = x[k];
+            for (int j = child[k + 1] - 1; j >= child[k]; --j) r -= factor[j] * x[j];
+            x[k] = r;
         }
         __syncthreads();
     }
+    for (int k = threadIdx.x; k < a.n; k += blockDim.x) x[k] /= a.diag[k];
+    __syncthreads();
+    for (int L = 1; L < a.n_levels; ++L) {
+        for (int k = off[L] + threadIdx.x; k < off[L + 1]; k += blockDim.x)
+            x[k] -= up[k] * x[parent[k]];
+        __syncthreads();
+    }
+    for (int k = threadIdx.x; k < a.n; k += blockDim.x) a.vm[a.order[k]] = x[k];
 }
 
 // evaluateCoupling: I = (Vnet - Vtissue) / R_pvj per terminal and its
@@ -142,15 +195,16 @@ struct cfg_purkinje {
     int root = 0;
     double root_start = 1e300, root_duration = 0, root_intensity = 0;
     // graph, host
-    std::vector<int> ea, eb, parent, order, rev, level_off, child_off, children, term_node,
+    std::vector<int> ea, eb, parent, pos_parent, order, level_off, child, term_node,
         term_off, term_idx;
     std::vector<double> elen, econd, term_loc;
     // device
-    int *d_level_off = nullptr, *d_order = nullptr, *d_parent = nullptr, *d_child_off = nullptr,
-        *d_children = nullptr, *d_term_off = nullptr, *d_term_idx = nullptr,
+    int *d_level_off = nullptr, *d_level = nullptr, *d_order = nullptr, *d_parent = nullptr, *d_child = nullptr,
+        *d_term_off = nullptr, *d_term_idx = nullptr,
         *d_term_node = nullptr;
-    double *d_vm = nullptr, *d_iion = nullptr, *d_diag0 = nullptr, *d_pc = nullptr,
-           *d_cc = nullptr, *d_diag = nullptr, *d_rhs = nullptr, *d_term_current = nullptr;
+    double *d_vm = nullptr, *d_iion = nullptr, *d_factor = nullptr, *d_up = nullptr,
+           *d_diag = nullptr, *d_rhs = nullptr, *d_term_current = nullptr;
+    int block = kPkBlock;
     double prepared_dt = 0.0;
     // coupling to a monodomain context
     cfg_monodomain* md = nullptr;
@@ -171,11 +225,11 @@ namespace {
 void pk_free(cfg_purkinje* pk)
 {
     if (pk->stream) cudaStreamSynchronize(pk->stream);
-    for (int** p : {&pk->d_level_off, &pk->d_order, &pk->d_parent, &pk->d_child_off,
-                    &pk->d_children, &pk->d_term_off, &pk->d_term_idx, &pk->d_term_node,
+    for (int** p : {&pk->d_level_off, &pk->d_level, &pk->d_order, &pk->d_parent, &pk->d_child,
+                    &pk->d_term_off, &pk->d_term_idx, &pk->d_term_node,
                     &pk->d_term_cell, &pk->d_dep_off, &pk->d_dep_term})
         dfree(*p);
-    for (double** p : {&pk->d_vm, &pk->d_iion, &pk->d_diag0, &pk->d_pc, &pk->d_cc, &pk->d_diag,
+    for (double** p : {&pk->d_vm, &pk->d_iion, &pk->d_factor, &pk->d_up, &pk->d_diag,
                        &pk->d_rhs, &pk->d_term_current, &pk->d_sphere_vol, &pk->d_dep_value,
                        &pk->d_src_total})
         dfree(*p);
@@ -224,12 +278,21 @@ int prepare_dt(cfg_purkinje* pk, double dt)
             cc[size_t(b)] = -coeffA;
         }
     }
-    CFG_CUDA_TRY(cudaMemcpyAsync(pk->d_diag0, diag.data(), n * sizeof(double),
-                                 cudaMemcpyHostToDevice, pk->stream));
-    CFG_CUDA_TRY(cudaMemcpyAsync(pk->d_pc, pc.data(), n * sizeof(double), cudaMemcpyHostToDevice,
-                                 pk->stream));
-    CFG_CUDA_TRY(cudaMemcpyAsync(pk->d_cc, cc.data(), n * sizeof(double), cudaMemcpyHostToDevice,
-                                 pk->stream));
+    // elimination, children before parents, and the arrays by position
+    std::vector<double> factor(n, 0.0), up(n, 0.0), pos_diag(n, 1.0);
+    for (size_t k = n; k-- > 0;) {
+        const size_t c = size_t(pk->order[k]);
+        pos_diag[k] = diag[c];
+        if (k == 0) break;
+        factor[k] = cc[c] / diag[c];
+        up[k] = pc[c] / diag[c];
+        double& d = diag[size_t(pk->parent[c])];
+        d = std::fma(-factor[k], pc[c], d);
+    }
+    for (const auto& v : {std::make_pair(pk->d_factor, &factor), std::make_pair(pk->d_up, &up),
+                          std::make_pair(pk->d_diag, &pos_diag)})
+        CFG_CUDA_TRY(cudaMemcpyAsync(v.first, v.second->data(), n * sizeof(double),
+                                     cudaMemcpyHostToDevice, pk->stream));
     CFG_CUDA_TRY(cudaStreamSynchronize(pk->stream));
     pk->prepared_dt = dt;
     return CFG_OK;
@@ -241,37 +304,40 @@ int advance(cfg_purkinje* pk, double t0, double dt)
     if (dt != pk->prepared_dt)
         if (int rc = prepare_dt(pk, dt)) return rc;
     if (int rc = cfg_ionic_solve_device(pk->ion, t0, dt / 2.0, pk->d_vm, pk->d_iion)) return rc;
-    PkRhsArgs r{};
-    r.n = pk->n;
-    r.dt = dt;
-    r.chicm = pk->chi * pk->cm;
-    r.t0 = t0;
-    r.root = pk->root;
-    r.root_start = pk->root_start;
-    r.root_end = pk->root_start + pk->root_duration;
-    r.root_intensity = pk->root_intensity;
-    r.term_off = pk->d_term_off;
-    r.term_idx = pk->d_term_idx;
-    r.term_current = pk->d_term_current;
-    r.vm = pk->d_vm;
-    r.iion = pk->d_iion;
-    r.diag0 = pk->d_diag0;
-    r.diag = pk->d_diag;
-    r.rhs = pk->d_rhs;
-    k_pk_rhs<<<unsigned((pk->n + 255) / 256), 256, 0, pk->stream>>>(r);
-    HinesArgs h{};
-    h.n_levels = int(pk->level_off.size()) - 1;
-    h.level_off = pk->d_level_off;
-    h.order = pk->d_order;
-    h.parent = pk->d_parent;
-    h.child_off = pk->d_child_off;
-    h.children = pk->d_children;
-    h.pc = pk->d_pc;
-    h.cc = pk->d_cc;
-    h.diag = pk->d_diag;
-    h.rhs = pk->d_rhs;
-    h.vm = pk->d_vm;
-    k_pk_hines<<<1, kPkBlock, 0, pk->stream>>>(h);
+    CableArgs a{};
+    a.n = int(pk->n);
+    a.n_levels = int(pk->level_off.size()) - 1;
+    a.dt = dt;
+    a.chicm = pk->chi * pk->cm;
+    a.t0 = t0;
+    a.root = pk->root;
+    a.root_start = pk->root_start;
+    a.root_end = pk->root_start + pk->root_duration;
+    a.root_intensity = pk->root_intensity;
+    a.term_off = pk->d_term_off;
+    a.term_idx = pk->d_term_idx;
+    a.term_current = pk->d_term_current;
+    a.iion = pk->d_iion;
+    a.vm = pk->d_vm;
+    a.level_off = pk->d_level_off;
+    a.level = pk->d_level;
+    a.order = pk->d_order;
+    a.parent = pk->d_parent;
+    a.child = pk->d_child;
+    a.factor = pk->d_factor;
+    a.up = pk->d_up;
+    a.diag = pk->d_diag;
+    a.rhs = pk->d_rhs;
+    const size_t bytes = cable_bytes(size_t(pk->n), size_t(a.n_levels));
+    if (bytes <= kCableShared) {
+        if (bytes > 48 * 1024)
+            CFG_CUDA_TRY(cudaFuncSetAttribute(k_pk_cable<true>,
+                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              int(kCableShared)));
+        k_pk_cable<true><<<1, pk->block, bytes, pk->stream>>>(a);
+    } else {
+        k_pk_cable<false><<<1, pk->block, 0, pk->stream>>>(a);
+    }
     CFG_CUDA_TRY(cudaGetLastError());
     return cfg_ionic_solve_device(pk->ion, t0 + (dt / 2.0), dt / 2.0, pk->d_vm, pk->d_iion);
 }
@@ -403,28 +469,36 @@ int cfg_purkinje_create(const cfg_purkinje_desc* d, cfg_purkinje** out)
         return fail(CFG_ERR_INVALID, "Conduction graph is not connected: BFS from node 0 "
                                      "reached %lld of %lld nodes.", tail, n);
     }
-    pk->rev.assign(pk->order.rbegin(), pk->order.rend());
     // BFS order is sorted by depth: the levels are its ranges
     pk->level_off.push_back(0);
     for (long long k = 1; k < n; ++k)
         if (depth[size_t(pk->order[size_t(k)])] != depth[size_t(pk->order[size_t(k - 1)])])
             pk->level_off.push_back(int(k));
     pk->level_off.push_back(int(n));
-    // children of each node in reverse BFS order (the elimination's order)
-    pk->child_off.assign(size_t(n) + 1, 0);
-    for (long long k = 0; k < n; ++k) {
-        const int p = pk->parent[size_t(pk->rev[size_t(k)])];
-        if (p >= 0) pk->child_off[size_t(p) + 1]++;
-    }
-    for (long long i = 0; i < n; ++i) pk->child_off[size_t(i) + 1] += pk->child_off[size_t(i)];
-    pk->children.assign(size_t(std::max<long long>(n - 1, 1)), 0);
+    // by position: parents, and the first child of each (BFS order keeps the
+    // children of a node together, in the order of their parents)
     {
-        std::vector<int> f(size_t(n), 0);
-        for (long long k = 0; k < n; ++k) {
-            const int c = pk->rev[size_t(k)], p = pk->parent[size_t(c)];
-            if (p >= 0) pk->children[size_t(pk->child_off[size_t(p)] + f[size_t(p)]++)] = c;
+        std::vector<int> at(static_cast<size_t>(n));
+        for (long long k = 0; k < n; ++k) at[size_t(pk->order[size_t(k)])] = int(k);
+        pk->pos_parent.assign(size_t(n), 0);
+        pk->child.assign(size_t(n) + 1, 1);
+        for (long long k = 1; k < n; ++k) {
+            const int q = at[size_t(pk->parent[size_t(pk->order[size_t(k)])])];
+            pk->pos_parent[size_t(k)] = q;
+            pk->child[size_t(q) + 1] = int(k) + 1;
         }
+        for (long long k = 1; k <= n; ++k)
+            pk->child[size_t(k)] = std::max(pk->child[size_t(k)], pk->child[size_t(k - 1)]);
     }
+    // a thread per node, or per node of the widest level, as far as a block has them
+    int widest = 1;
+    std::vector<int> level(static_cast<size_t>(n));
+    for (size_t L = 0; L + 1 < pk->level_off.size(); ++L) {
+        widest = std::max(widest, pk->level_off[L + 1] - pk->level_off[L]);
+        for (int k = pk->level_off[L]; k < pk->level_off[L + 1]; ++k) level[size_t(k)] = int(L);
+    }
+    const long long threads = n <= kPkBlock ? n : std::min(kPkBlock, std::max(128, widest));
+    pk->block = int((threads + 31) / 32 * 32);
     // terminals per node, in terminal order
     pk->term_node.assign(d->pvj_nodes, d->pvj_nodes + d->n_pvj);
     pk->term_loc.assign(d->pvj_locations, d->pvj_locations + 3 * d->n_pvj);
@@ -461,15 +535,15 @@ int cfg_purkinje_create(const cfg_purkinje_desc* d, cfg_purkinje** out)
     std::vector<double> v0(size_t(n), vm_rest), zero(size_t(std::max(d->n_pvj, 1)), 0.0);
     if (!e) e = upload(&pk->d_level_off, pk->level_off);
     if (!e) e = upload(&pk->d_order, pk->order);
-    if (!e) e = upload(&pk->d_parent, pk->parent);
-    if (!e) e = upload(&pk->d_child_off, pk->child_off);
-    if (!e) e = upload(&pk->d_children, pk->children);
+    if (!e) e = upload(&pk->d_level, level);
+    if (!e) e = upload(&pk->d_parent, pk->pos_parent);
+    if (!e) e = upload(&pk->d_child, pk->child);
     if (!e) e = upload(&pk->d_term_off, pk->term_off);
     if (!e) e = upload(&pk->d_term_idx, pk->term_idx);
     if (!e) e = upload(&pk->d_term_node, pk->term_node);
     if (!e) e = upload(&pk->d_vm, v0);
     if (!e) e = upload(&pk->d_term_current, zero);
-    for (double** p : {&pk->d_iion, &pk->d_diag0, &pk->d_pc, &pk->d_cc, &pk->d_diag, &pk->d_rhs})
+    for (double** p : {&pk->d_iion, &pk->d_factor, &pk->d_up, &pk->d_diag, &pk->d_rhs})
         if (!e) e = dmalloc(p, size_t(n));
     if (!e) e = cudaMemset(pk->d_iion, 0, size_t(n) * sizeof(double));
     if (e) return bail(fail(CFG_ERR_CUDA, "network allocation: %s", cudaGetErrorString(e)));
