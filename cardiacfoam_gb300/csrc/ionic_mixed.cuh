@@ -102,21 +102,41 @@ CFG_D __forceinline__ void add_wide(float& hi, float& lo, float d)
     hi = h;
 }
 
+// The accepted state from a loop that is not unrolled.  Unrolled, the compiler
+// shares the error norm's y5 = fma(h, q, y0) and rounded increment with the update;
+// the same values here keep the roundings of both forms alike.
+CFG_D __forceinline__ float accept_narrow(float y, float h, float q)
+{
+    return __fmaf_rn(h, q, y);
+}
+
+CFG_D __forceinline__ void accept_wide(float& hi, float& lo, float h, float q)
+{
+    const float s = __fmaf_rn(h, q, hi), d = __fmul_rn(h, q);
+    const float bp = __fsub_rn(s, hi);
+    const float err = __fadd_rn(__fsub_rn(hi, __fsub_rn(s, bp)), __fsub_rn(d, bp));
+    const float l = __fadd_rn(lo, err);
+    hi = __fadd_rn(s, l);
+    lo = __fsub_rn(l, __fsub_rn(hi, s));
+}
+
 // Stage input T = Y + h * sum_j a_sj k_j for stages 2..5 (s = 1..4); T is
 // the stage's own slot K + s P, where its derivative is then evaluated in
 // place.
-template <class M>
-CFG_D __forceinline__ void stage_input(int s, float h, const float (&Y)[M::NS], float* T,
-                                       const float* K)
+// Y is an array of registers, with loops unrolled all the way (U = NS), or a
+// pointer, with any U.  (The stage-6 sums stay unrolled: as a loop they gain 12 %
+// but the compiler fuses their products otherwise.)
+template <class M, int U, class YT>
+CFG_D __forceinline__ void stage_input(int s, float h, const YT& Y, float* T, const float* K)
 {
     constexpr int NS = M::NS, P = Slice<M>::NSP;
     switch (s) {
     case 1:
-#pragma unroll
+#pragma unroll U
         for (int i = 0; i < NS; ++i) T[i] = Y[i] + h * (fa21 * K[i]);
         break;
     case 2:
-#pragma unroll
+#pragma unroll U
         for (int i = 0; i < NS; ++i) {
             float acc = fa31 * K[i];
             acc += fa32 * K[P + i];
@@ -124,7 +144,7 @@ CFG_D __forceinline__ void stage_input(int s, float h, const float (&Y)[M::NS], 
         }
         break;
     case 3:
-#pragma unroll
+#pragma unroll U
         for (int i = 0; i < NS; ++i) {
             float acc = fa41 * K[i];
             acc += fa42 * K[P + i];
@@ -133,7 +153,7 @@ CFG_D __forceinline__ void stage_input(int s, float h, const float (&Y)[M::NS], 
         }
         break;
     default:
-#pragma unroll
+#pragma unroll U
         for (int i = 0; i < NS; ++i) {
             float acc = fa51 * K[i];
             acc += fa52 * K[P + i];
@@ -148,8 +168,8 @@ CFG_D __forceinline__ void stage_input(int s, float h, const float (&Y)[M::NS], 
 // Stage-6 input into slot 3 (k4's, read first), and P, E and the round-off
 // bound of E into slots 1, 2, 4 (k2 and the old k3..k5 are not needed
 // afterwards: b2 = e2 = 0).
-template <class M>
-CFG_D __forceinline__ void stage6_input(float h, const float (&Y)[M::NS], float* T, float* K)
+template <class M, class YT>
+CFG_D __forceinline__ void stage6_input(float h, const YT& Y, float* T, float* K)
 {
     constexpr int NS = M::NS, P = Slice<M>::NSP;
 #pragma unroll
@@ -178,6 +198,12 @@ CFG_D __forceinline__ void stage6_input(float h, const float (&Y)[M::NS], float*
 // State i of Y at a run-time index (for failure records), without indexing
 // the register array at run time.
 template <int NS>
+CFG_D __forceinline__ double state_at(const float* const& Y, int i)
+{
+    return double(Y[i]);
+}
+
+template <int NS>
 CFG_D __forceinline__ double state_at(const float (&Y)[NS], int i)
 {
     float v = 0.0f;
@@ -187,9 +213,8 @@ CFG_D __forceinline__ double state_at(const float (&Y)[NS], int i)
     return double(v);
 }
 
-template <class M, bool SV, class KS>
-CFG_D __forceinline__ long long solve(double xs, double xe, float D, float (&Y)[M::NS], float* K,
-                                      float (&LO)[Slice<M>::NWA],
+template <class M, bool SV, int U, class KS, class YT, class LT>
+CFG_D __forceinline__ long long solve(double xs, double xe, float D, YT& Y, float* K, LT& LO,
                                       float& dx_try, const KS& Kc, int tissue,
                                       const CfgStimulus& st, const OdeSettings& s,
                                       unsigned& evals, IonicFailure& why, float& iion,
@@ -218,7 +243,7 @@ CFG_D __forceinline__ long long solve(double xs, double xe, float D, float (&Y)[
                 // the last accepted substep, as ODESolver reports it
                 why.reason = 1;
                 why.x = xs + double(u_prev); why.dx = dx; why.err = err; why.worst = worst;
-                why.value = worst >= 0 ? state_at(Y, worst) : 0.0;
+                why.value = worst >= 0 ? state_at<M::NS>(Y, worst) : 0.0;
                 why.steps = n - 1;
                 return -1;
             }
@@ -238,18 +263,18 @@ CFG_D __forceinline__ long long solve(double xs, double xe, float D, float (&Y)[
         if (sg == 0) {
             // k1 = f(y), evaluated in slot 0 from a copy of y
             out = K;
-#pragma unroll
+#pragma unroll U
             for (int i = 0; i < NS; ++i) out[i] = Y[i];
         } else if (sg < 5) {
             out = K + sg * P;
-            stage_input<M>(sg, h, Y, out, K);
+            stage_input<M, U>(sg, h, Y, out, K);
         } else if (sg == 5) {
             out = K + 3 * P;
             stage6_input<M>(h, Y, out, K);
         } else {
             // the current at the end, from y in a free slot
             out = K + P;
-#pragma unroll
+#pragma unroll U
             for (int i = 0; i < NS; ++i) out[i] = Y[i];
         }
         const float* in = out;
@@ -275,7 +300,7 @@ CFG_D __forceinline__ long long solve(double xs, double xe, float D, float (&Y)[
         float maxerr = 0.0f;
         bool finite = true;
         worst = -1;
-#pragma unroll
+#pragma unroll U
         for (int i = 0; i < NS; ++i) {
             const float k6 = K[3 * P + i];
             const float y0 = Y[i];
@@ -299,7 +324,7 @@ CFG_D __forceinline__ long long solve(double xs, double xe, float D, float (&Y)[
             if (!(dx >= 1e-37f)) {
                 why.reason = 2;
                 why.x = xs + double(u); why.dx = dx; why.err = err; why.worst = worst;
-                why.value = worst >= 0 ? state_at(Y, worst) : 0.0;
+                why.value = worst >= 0 ? state_at<M::NS>(Y, worst) : 0.0;
                 why.steps = n;
                 return -1;
             }
@@ -308,8 +333,16 @@ CFG_D __forceinline__ long long solve(double xs, double xe, float D, float (&Y)[
         }
         // --- accept: y = y5 (slow states as hi + lo)
         int w = 0;
-#pragma unroll
+#pragma unroll U
         for (int i = 0; i < NS; ++i) {
+            if constexpr (U < NS) {
+                const float q = __fmaf_rn(fb6, K[3 * P + i], K[P + i]);
+                if (is_wide<M::WIDE_MASK>(i))
+                    accept_wide(Y[i], LO[w++], h, q);
+                else
+                    Y[i] = accept_narrow(Y[i], h, q);
+                continue;
+            }
             const float incr = h * (K[P + i] + fb6 * K[3 * P + i]);
             if (is_wide<M::WIDE_MASK>(i)) {
                 float hi = Y[i], lo = LO[w];
@@ -399,7 +432,7 @@ ionic_mixed_kernel(IonicLaunch p)
         if constexpr (TISSUE > 0) {
             const ConstFold<float, M, TISSUE> Kc{};
             if constexpr (!SV) M::template hoist_vm<float>(Y[0], Kc, TISSUE, H.v);
-            nsub = mixed::solve<M, SV>(ts, te, float(dtm), Y, K, LO, dx_try, Kc, TISSUE, p.stim,
+            nsub = mixed::solve<M, SV, M::NS>(ts, te, float(dtm), Y, K, LO, dx_try, Kc, TISSUE, p.stim,
                                        p.ode, evals, why, iion, H.v);
         } else {
             const int tissue = p.tissue_cell ? int(p.tissue_cell[c]) : p.tissue;
@@ -415,7 +448,7 @@ ionic_mixed_kernel(IonicLaunch p)
             M::init(C, yinit, tissue, scp);
             const ConstView<float> Kc{C};
             if constexpr (!SV) M::template hoist_vm<float>(Y[0], Kc, tissue, H.v);
-            nsub = mixed::solve<M, SV>(ts, te, float(dtm), Y, K, LO, dx_try, Kc, tissue, p.stim,
+            nsub = mixed::solve<M, SV, M::NS>(ts, te, float(dtm), Y, K, LO, dx_try, Kc, tissue, p.stim,
                                        p.ode, evals, why, iion, H.v);
         }
         if (nsub < 0) {
