@@ -724,20 +724,23 @@ static FastDiv make_fastdiv(unsigned d)
 }
 
 // rows of a general mesh are visited over the full ELL width when it is 4
-// (tetrahedra) or 6 (hexahedra)
-static void* coop_kernel(bool pair, bool nc_fp32, int w)
+// (tetrahedra) or 6 (hexahedra); CR is the type the explicit correction's
+// arrays are kept in, by the ionic form and not by the PCG's arithmetic
+template <class CR>
+static void* coop_kernel_of(bool pair, int w)
 {
     if (pair)
-        return w == 4   ? (void*)k_implicit_pair<float, 4>
-               : w == 6 ? (void*)k_implicit_pair<float, 6>
-                        : (void*)k_implicit_pair<float, 0>;
-    if (nc_fp32)
-        return w == 4   ? (void*)k_implicit_coop<float, 4>
-               : w == 6 ? (void*)k_implicit_coop<float, 6>
-                        : (void*)k_implicit_coop<float, 0>;
-    return w == 4   ? (void*)k_implicit_coop<double, 4>
-           : w == 6 ? (void*)k_implicit_coop<double, 6>
-                    : (void*)k_implicit_coop<double, 0>;
+        return w == 4   ? (void*)k_implicit_pair<CR, 4>
+               : w == 6 ? (void*)k_implicit_pair<CR, 6>
+                        : (void*)k_implicit_pair<CR, 0>;
+    return w == 4   ? (void*)k_implicit_coop<CR, 4>
+           : w == 6 ? (void*)k_implicit_coop<CR, 6>
+                    : (void*)k_implicit_coop<CR, 0>;
+}
+
+static void* coop_kernel(bool pair, bool nc_fp32, int w)
+{
+    return nc_fp32 ? coop_kernel_of<float>(pair, w) : coop_kernel_of<double>(pair, w);
 }
 
 // Block size and grid of a kernel for n rows, one block per SM: the smallest
