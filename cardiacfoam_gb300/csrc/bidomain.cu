@@ -690,6 +690,19 @@ struct PairStep {
     }
 };
 
+// The power of two that brings a value near one, between 2^-126 and 2^126, and
+// the exact product of a pair with it.
+__device__ __forceinline__ float unit_scale(fp::P v)
+{
+    const int e = int((__float_as_uint(v.x) >> 23) & 0xffu);   // 127 for [1, 2)
+    return __uint_as_float(unsigned(max(1, min(253, 254 - e))) << 23);
+}
+
+__device__ __forceinline__ fp::P scaled(fp::P a, float s)
+{
+    return fp::make(__fmul_rn(a.x, s), __fmul_rn(a.y, s));
+}
+
 // The solve where every row has a thread (one block per SM): a row's matrix
 // entries, its neighbours' preconditioner and its x, p, r, s and w stay in
 // registers for the whole solve, and only r, s and w are published.  What
@@ -697,7 +710,9 @@ struct PairStep {
 // of pair divisions, and the neighbours' values.  So these are loaded as soon
 // as the blocks have met, before the totals are formed, and the reciprocals
 // that beta and (p, A p) need are formed in the iteration before, which leaves
-// one division in the chain.  A step of 427 phiE iterations on 64,000 rows
+// one division in the chain.  (z, r) falls with the square of the residual and
+// may leave the range whose reciprocals floats hold, so it is scaled by the
+// power of two that brings it near one: exact, and beta stays what it is.  A step of 427 phiE iterations on 64,000 rows
 // takes 2.58 ms where the strided form below takes 2.86 (both in blocks of
 // 448), one of 326 on 8,000 rows 1.39 against 1.85 (blocks of 128).
 // Tried without gain: the block's own rows exchanged through shared memory.
@@ -765,7 +780,9 @@ __global__ void __launch_bounds__(B, 1) k_pcg_pair_row(CoopPcgArgs ca, PairPcgAr
         P s2[2] = {live ? fp::add(fp::abs(fp::sub(ax, pa)), fp::abs(fp::sub(b, pa))) : zero,
                    live ? fp::mul(u, r) : zero};
         if (!sum(s2, Nothing())) { aborted = true; break; }
-        const P normf = fp::add(s2[0], small), inv_normf = fp::div(one, normf);
+        const P normf = fp::add(s2[0], small);
+        const float normf_unit = unit_scale(normf);
+        const P inv_normf = fp::div(one, scaled(normf, normf_unit));
         init_res = fp::div(s1[1], normf);
         const P rel_init = fp::mul(rel, init_res);
         const auto conv = [&](P rr) {
@@ -794,18 +811,20 @@ __global__ void __launch_bounds__(B, 1) k_pcg_pair_row(CoopPcgArgs ca, PairPcgAr
         };
         if (!sum(s3, gather)) { aborted = true; break; }
         P gamma = s2[1], delta = s3[0], s = zero, p = zero;
-        P inv_gamma_old = zero, inv_alpha_old = zero;
+        P inv_gamma_old = zero, inv_alpha_old = zero;   // of the scaled gamma
+        float unit_old = 1.0f;
         for (;;) {
             // (p, A p) = delta - beta gamma / alpha_old
             PairStep ps;
             ps.first = iter == 0;
-            ps.beta = fp::mul(gamma, inv_gamma_old);
+            ps.beta = fp::mul(scaled(gamma, unit_old), inv_gamma_old);
             const P pap = fp::sub(delta, fp::mul(fp::mul(ps.beta, gamma), inv_alpha_old));
             if (pap.x == 0.0f) break;   // checkSingularity
             ps.alpha = fp::div(gamma, pap);
             ps.nalpha = fp::neg(ps.alpha);
-            inv_gamma_old = fp::div(one, gamma);
-            inv_alpha_old = fp::mul(pap, inv_gamma_old);
+            unit_old = unit_scale(gamma);
+            inv_gamma_old = fp::div(one, scaled(gamma, unit_old));
+            inv_alpha_old = fp::mul(scaled(pap, unit_old), inv_gamma_old);
             s = ps.s_next(w, s);
             const P u_old = fp::mul(rd, r);
             p = ps.first ? u_old : fp::madd(ps.beta, p, u_old);
@@ -827,7 +846,7 @@ __global__ void __launch_bounds__(B, 1) k_pcg_pair_row(CoopPcgArgs ca, PairPcgAr
             P s4[3] = {live ? fp::mul(un, r) : zero, live ? fp::mul(w, un) : zero,
                        live ? fp::abs(r) : zero};
             if (!sum(s4, gather)) { aborted = true; break; }
-            res = fp::mul(s4[2], inv_normf);
+            res = fp::mul(scaled(s4[2], normf_unit), inv_normf);
             ++iter;
             if (conv(res) || iter >= max_iter) {
                 if (!conv(res)) status = 1;
