@@ -80,15 +80,18 @@ CFG_HD __forceinline__ double cfg_fma(double a, double b, double c)
 // a / b by the reciprocal r = RN(1 / b) at hand: the product, corrected once by
 // its exact remainder, which is the correctly rounded quotient but for rare
 // ties (Markstein 1990), in three instructions where the general division
-// takes about nine.  A quotient that is not finite is passed on as it is (the
-// correction would turn an infinity into a NaN).
+// takes about nine.  A quotient that is not finite, and the zero that an
+// infinite b leaves (r = 0), are passed on as they are: the correction would
+// turn them into a NaN.  r's bits are tested, which takes no FP64 instruction.
+// Where b is so small that r overflows (below 2^-1024), the quotient does too.
 CFG_HD __forceinline__ double cfg_quotient(double a, double b, double r)
 {
     const double q = a * r;
 #ifdef __CUDA_ARCH__
-    if ((__double2hiint(q) & 0x7ff00000) == 0x7ff00000) return q;
+    if ((__double2hiint(q) & 0x7ff00000) == 0x7ff00000 || (__double2hiint(r) & 0x7fffffff) == 0)
+        return q;
 #else
-    if (!std::isfinite(q)) return q;
+    if (!std::isfinite(q) || r == 0.0) return q;
 #endif
     return cfg_fma(cfg_fma(-q, b, a), r, q);
 }
