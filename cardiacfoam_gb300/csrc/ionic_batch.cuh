@@ -198,21 +198,22 @@ __global__ void __launch_bounds__(128) batch_fp64_kernel(BatchLaunch p)
     }
 }
 
-// Mixed form: FP32 arithmetic, slow states as (hi, lo) pairs, stage data in shared
-// memory (see ionic_mixed.cuh); the state in registers (REG) or beside the stage
-// data.
+// Mixed form: FP32 arithmetic, slow states as (hi, lo) pairs, the state and the
+// stage data in shared memory (see ionic_mixed.cuh).
 //
 // What bounds it is the fetch of instructions: with a warp or two on an SM
 // partition nothing hides it, and the loops over the states, unrolled for a state
 // in registers, are as long as the right-hand side (half of a warp's time went to
 // it for 16,384 ToRORd cells).  With the state in shared memory they are loops.
 // 300 steps of those cells take 34.4 ms instead of 55.1, 100 steps of 65,536 cells
-// 74.9 instead of 91.9 (TNNP 37.9 for 43.1).  While every warp has an SM's
-// instruction cache to itself, registers are 2 % faster (batch_launch).
-template <class M, bool REG>
+// 74.9 instead of 91.9 (TNNP 37.9 for 43.1).  Up to a warp per SM the registers'
+// form is 1 % (TNNP) to 3 % (ORd) faster, and 1 to 8 % slower in the other models;
+// it rounds otherwise in places, and a cell's result must not depend on how many
+// others there are, so every population takes this form.
+template <class M>
 struct BatchSlice {
     using S = mixed::Slice<M>;
-    static constexpr int len = REG ? S::len : (S::raw + S::NSP + S::NW) | 1;   // stages, Y, LO
+    static constexpr int len = (S::raw + S::NSP + S::NW) | 1;   // stages, Y, LO
     static constexpr int block =
         32 * mixed::blocks_per_sm(32, len) > 64 * mixed::blocks_per_sm(64, len) ? 32 : 64;
     static constexpr int fit = mixed::blocks_per_sm(block, len);
@@ -225,12 +226,17 @@ struct BatchSlice {
     static constexpr int smem_bytes = block * len * 4;
 };
 
-template <class M, int T, int U, class YT, class LT>
-CFG_D __forceinline__ void batch_mixed(const BatchLaunch& p, float* K, YT& Y, LT& LO)
+template <class M, int T>
+__global__ void __launch_bounds__(BatchSlice<M>::block, BatchSlice<M>::min_blocks)
+batch_mixed_kernel(BatchLaunch p)
 {
     using S = mixed::Slice<M>;
     using L = Layout<M, false>;
-    constexpr int NS = M::NS, P = S::NSP;
+    constexpr int NS = M::NS, P = S::NSP, U = 4;
+    extern __shared__ float cfg_batch_smem[];
+    float* K = cfg_batch_smem + threadIdx.x * BatchSlice<M>::len;
+    float* Y = K + S::raw;
+    float* LO = Y + S::NSP;
     unsigned evals = 0;
     for (;;) {
         const long long c = (long long)atomicAdd(p.queue, 1ull);
@@ -313,24 +319,6 @@ CFG_D __forceinline__ void batch_mixed(const BatchLaunch& p, float* K, YT& Y, LT
         unsigned long long v = evals;
         for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
         if ((threadIdx.x & 31) == 0 && v) atomicAdd(p.rhs_evals, v);
-    }
-}
-
-template <class M, int T, bool REG>
-__global__ void __launch_bounds__(BatchSlice<M, REG>::block, BatchSlice<M, REG>::min_blocks)
-batch_mixed_kernel(BatchLaunch p)
-{
-    using S = mixed::Slice<M>;
-    extern __shared__ float cfg_batch_smem[];
-    float* K = cfg_batch_smem + threadIdx.x * BatchSlice<M, REG>::len;
-    if constexpr (REG) {
-        float Y[M::NS];
-        float LO[S::NWA];
-        batch_mixed<M, T, M::NS>(p, K, Y, LO);
-    } else {
-        float* Y = K + S::raw;
-        float* LO = Y + S::NSP;
-        batch_mixed<M, T, 4>(p, K, Y, LO);
     }
 }
 

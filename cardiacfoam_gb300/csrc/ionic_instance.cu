@@ -167,8 +167,8 @@ extern "C" void CFG_CAT3(cfg_ionic_host_init_, CFG_MODEL, )(double* C, double* y
 
 // ---------------------------------------------------------------- batched single cells
 
-template <int T, bool REG>
-static cudaError_t batch_launch_form(const cfg::BatchLaunch& p, int sms, cudaStream_t s)
+template <int T>
+static cudaError_t batch_launch(const cfg::BatchLaunch& p, cudaStream_t s)
 {
     int block, smem;
     void (*fn)(cfg::BatchLaunch);
@@ -177,14 +177,17 @@ static cudaError_t batch_launch_form(const cfg::BatchLaunch& p, int sms, cudaStr
         block = 128;
         smem = 0;
     } else {
-        fn = cfg::batch_mixed_kernel<M, T, REG>;
-        block = cfg::BatchSlice<M, REG>::block;
-        smem = cfg::BatchSlice<M, REG>::smem_bytes;
+        fn = cfg::batch_mixed_kernel<M, T>;
+        block = cfg::BatchSlice<M>::block;
+        smem = cfg::BatchSlice<M>::smem_bytes;
     }
     // persistent grid: every block resident, cells handed out by the queue
-    static int per_sm = 0;
+    static int per_sm = 0, sms = 0;
     if (!per_sm) {
-        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, block, smem);
+        int dev = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (!e) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (!e) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, block, smem);
         if (e) return e;
         if (per_sm < 1) per_sm = 1;
     }
@@ -193,28 +196,6 @@ static cudaError_t batch_launch_form(const cfg::BatchLaunch& p, int sms, cudaStr
     const unsigned grid = unsigned(want < cap ? want : cap);
     fn<<<grid, block, smem, s>>>(p);
     return cudaGetLastError();
-}
-
-template <int T>
-static cudaError_t batch_launch(const cfg::BatchLaunch& p, cudaStream_t s)
-{
-    static int sms = 0;
-    if (!sms) {
-        int dev = 0;
-        cudaError_t e = cudaGetDevice(&dev);
-        if (!e) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (e) return e;
-    }
-    if constexpr (!kFP64) {
-        // State in registers while few warps share an SM's instruction cache: up to
-        // a warp per SM (ToRORd, 60 steps: 500 cells 7.77 ms against 8.00 in shared
-        // memory, 4,800 cells 9.76 against 9.59, 13,000 cells 16.3 against 12.2), for
-        // small models up to a warp per partition (TNNP: 13,000 cells 11.45 against
-        // 11.60; 100 steps of 65,536 cells 43.1 against 37.9).
-        const bool reg = p.n <= (M::NS > 20 ? 32LL : 128LL) * sms;
-        if (reg) return batch_launch_form<T, true>(p, sms, s);
-    }
-    return batch_launch_form<T, false>(p, sms, s);
 }
 
 template <int T0, int... TR>
@@ -233,12 +214,9 @@ static cudaError_t batch_prepare(TissueList<TS...>)
         return cudaSuccess;
     } else {
         cudaError_t r[] = {cudaSuccess,
-                           cudaFuncSetAttribute(&cfg::batch_mixed_kernel<M, TS, true>,
+                           cudaFuncSetAttribute(&cfg::batch_mixed_kernel<M, TS>,
                                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                cfg::BatchSlice<M, true>::smem_bytes)...,
-                           cudaFuncSetAttribute(&cfg::batch_mixed_kernel<M, TS, false>,
-                                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                cfg::BatchSlice<M, false>::smem_bytes)...};
+                                                cfg::BatchSlice<M>::smem_bytes)...};
         for (cudaError_t x : r)
             if (x) return x;
         return cudaSuccess;
