@@ -371,7 +371,7 @@ int ionic_autotune(cfg_ionic* ion, double t0, double dt, const double* t_dev, co
     cudaStreamSynchronize(s);
     cleanup();
     if (e) return fail(CFG_ERR_CUDA, "autotune failed: %s", cudaGetErrorString(e));
-    if (block_out) *block_out = best_b > 0 ? best_b : max_b;
+    if (block_out) *block_out = best_b;
     if (cpt_out) *cpt_out = best_c;
     if (ms_out) *ms_out = best / float(repeats > 0 ? repeats : 1);
     return CFG_OK;

@@ -93,10 +93,15 @@ int cfg_ionic_solve_device(cfg_ionic* ion, double t0, double dt, const double* v
  * step kernel - threads per block (32 .. the kernel's largest) x cells per
  * thread (1, 2, 4) - on scratch copies of the states with the given Vm
  * (device pointer; NULL = resting Vm) and keeps the fastest for this
- * context.  The results of a step do not depend on the launch shape. */
+ * context.  *block and *cells_per_thread are the shape kept, as
+ * cfg_ionic_set_launch takes it: block 0 where the FP64 form's own rule, which
+ * is among the candidates, was the fastest.  The results of a step do not
+ * depend on the launch shape. */
 int cfg_ionic_autotune(cfg_ionic* ion, double t0, double dt, const double* vm_dev,
                        int* block, int* cells_per_thread, float* ms_per_step);
-/* The same launch shape set directly (block 0 = the kernel's largest). */
+/* The same launch shape set directly.  block 0, the default: the mixed form's
+ * largest block; in FP64 the rule by the number of cells, which shares 32 cells
+ * between four warps where they do not fill the SMs. */
 int cfg_ionic_set_launch(cfg_ionic* ion, int block, int cells_per_thread);
 
 /* Number of states and their names (ioNumStates/ioStateNames,
