@@ -121,6 +121,29 @@ struct CfgSlot {
 };
 CFG_HD __forceinline__ double cfg_hdiv(double a, CfgSlot h) { return cfg_quotient(a, h.v, h.r); }
 
+// The largest |error| / tolerance of a trial step and its state, kept as
+// numerator and denominator (one FP64 division per trial instead of one per
+// state).  Ratios are compared exactly: compared by rounded products, the norm
+// would depend in its last bit on the order of the states, and so on how they
+// are dealt to warps.
+struct ErrorNorm {
+    double e = 0.0, tol = 1.0;
+    int state = -1;
+
+    // |a| / tol_a > e / tol: RN(e tol_a) and its remainder against the rest of
+    // |a| tol, each one multiply-add.  A NaN is never larger.
+    CFG_HD __forceinline__ bool below(double a, double tol_a) const
+    {
+        const double q = e * tol_a;
+        return cfg_fma(a, tol, -q) > cfg_fma(e, tol_a, -q);
+    }
+    CFG_HD __forceinline__ void take(double a, double tol_a, int i)
+    {
+        if (below(a, tol_a)) { e = a; tol = tol_a; state = i; }
+    }
+    CFG_HD __forceinline__ double value() const { return e / tol; }
+};
+
 template <int N, class R>
 CFG_HD __forceinline__ R cfg_ipow(R x)
 {

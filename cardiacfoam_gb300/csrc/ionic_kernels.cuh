@@ -169,6 +169,14 @@ static __constant__ double kRkfC[6] = {0.0, rkf::c2, rkf::c3, rkf::c4, rkf::c5, 
 constexpr double kFp32NoiseUlps = 64.0;
 
 
+// The larger of two magnitudes by their bits (an FP64 comparison takes the FP64
+// pipe); NaN if one is.
+CFG_D __forceinline__ double larger_magnitude(double a, double b)
+{
+    const double p = fabs(a), q = fabs(b);
+    return __double_as_longlong(p) > __double_as_longlong(q) ? p : q;
+}
+
 // One right-hand-side evaluation with Vm among the states.  Not inlined: the
 // stage loop and the final current evaluation share one copy of the (large)
 // model body, which keeps the kernel's instruction footprint to a single
@@ -191,10 +199,8 @@ struct Hoisted {
 // RKF45::solve inside, Vm among the states.  The six right-hand-side
 // evaluations of a trial step (dydx0 and stages 2..6) run through one loop, so
 // the model body is instantiated once.  Stage sums are accumulated left to
-// right exactly as the host code writes them; the error norm keeps its
-// largest quotient as numerator and denominator (one FP64 division per trial
-// instead of one per state).  Returns accepted substeps, or -1 on maxSteps
-// overflow / step underflow.
+// right exactly as the host code writes them.  Returns accepted substeps, or -1
+// on maxSteps overflow / step underflow.
 template <class M, class KS>
 CFG_D __forceinline__ long long rkf45_solve(double xs, double xe, double (&y)[M::NS],
                                             double& dx_try, double (*k)[M::NS], const KS& K,
@@ -245,20 +251,17 @@ CFG_D __forceinline__ long long rkf45_solve(double xs, double xe, double (&y)[M:
             s0 = 1;
             // 5th-order solution and the embedded error (RKF45::solve), then
             // ODESolver::normalizeError
-            double en = 0.0, et = 1.0;   // the largest |error| / tolerance
-            worst = -1;
+            ErrorNorm norm;
 #pragma unroll kStateUnroll
             for (int i = 0; i < NS; ++i) {
                 yt[i] = y[i] + dx * (b1 * k[0][i] + b3 * k[2][i] + b4 * k[3][i]
                                      + b5 * k[4][i] + b6 * k[5][i]);
                 const double e_i = dx * (e1 * k[0][i] + e3 * k[2][i] + e4 * k[3][i]
                                          + e5 * k[4][i] + e6 * k[5][i]);
-                const double a = fabs(y[i]), b = fabs(yt[i]);
-                const double tol = s.abs_tol + s.rel_tol * (a > b ? a : b);
-                const double e = fabs(e_i);
-                if (e * et > en * tol) { en = e; et = tol; worst = i; }
+                norm.take(fabs(e_i), s.abs_tol + s.rel_tol * larger_magnitude(y[i], yt[i]), i);
             }
-            err = en / et;
+            err = norm.value();
+            worst = norm.state;
             if (!(err > 1)) break;
             double scale = s.safe_scale * pow(err, -s.alpha_dec);
             if (scale < s.min_scale) scale = s.min_scale;
@@ -302,9 +305,8 @@ CFG_D __forceinline__ long long rkf45_solve(double xs, double xe, double (&y)[M:
 //
 //   * the linear gates of a tissue step follow their closed form
 //     (linear_gates.cuh): 15 multiply-adds for a gate's five stage values,
-//     where its stage sums and slopes cost about 85, and the error norm keeps
-//     its largest quotient as numerator and denominator, one division per
-//     trial instead of one per state;
+//     where its stage sums and slopes cost about 85, and the error norm takes
+//     one division per trial instead of one per state (ErrorNorm);
 //   * the stages, trials and substeps of a lane are one loop, so the lanes of
 //     a warp that need different numbers of them meet at the right-hand side;
 //   * where the tiles do not fill the partitions, four warps share a tile
@@ -315,8 +317,9 @@ CFG_D __forceinline__ long long rkf45_solve(double xs, double xe, double (&y)[M:
 //     and publishes them, so every warp follows the same path.
 //
 // Stage sums are accumulated left to right as the host code writes them, with
-// explicit multiply-adds (and no contraction by the compiler), so that a cell's
-// result does not depend on the launch shape.
+// explicit multiply-adds (and no contraction by the compiler), and the error
+// norm is the largest ratio exactly, so that a cell's result does not depend on
+// the launch shape.
 template <class M, bool SV>
 struct StepSplit {
     using T = TissueSplit<M>;
@@ -526,8 +529,7 @@ CFG_D __forceinline__ void fp64_tile(const IonicLaunch& p, const KS& K, int tiss
         if (__any_sync(kFull, at_end)) {
             // 5th-order solution and the embedded error (RKF45::solve), then
             // ODESolver::normalizeError
-            double en = 0.0, et = 1.0;   // the largest |error| / tolerance
-            int ew = -1;
+            ErrorNorm norm;
             if (at_end) {
 #pragma unroll
                 for (int i = 0; i < NS; ++i) {
@@ -546,13 +548,12 @@ CFG_D __forceinline__ void fp64_tile(const IonicLaunch& p, const KS& K, int tiss
                         e_i = dx * cfg_fma(e6, k6, cfg_fma(e5, k5, cfg_fma(e4, k4,
                                        cfg_fma(e3, k3, e1 * k1))));
                     }
-                    const double a = fabs(y[i]), b = fabs(yt[i]);
-                    const double tol = cfg_fma(s.rel_tol, a > b ? a : b, s.abs_tol);
-                    const double e = fabs(e_i);
-                    if (e * et > en * tol) { en = e; et = tol; ew = i; }
+                    norm.take(fabs(e_i),
+                              cfg_fma(s.rel_tol, larger_magnitude(y[i], yt[i]), s.abs_tol), i);
                 }
             }
-            double nerr = en / et, ndx = 0.0;
+            double nerr = norm.value(), ndx = 0.0;
+            int ew = norm.state;
             bool accept = false;
             if constexpr (W > 1) {
                 sh.err[P][lane] = nerr;
@@ -561,6 +562,7 @@ CFG_D __forceinline__ void fp64_tile(const IonicLaunch& p, const KS& K, int tiss
             }
             if (W == 1 || P == 0) {
                 if constexpr (W > 1) {
+                    // the largest rounded ratio is the largest ratio, rounded
 #pragma unroll
                     for (int q = 1; q < W; ++q)
                         if (sh.err[q][lane] > nerr) {
