@@ -39,7 +39,10 @@ mixed form takes the body apart at what depends on V and constants alone:
 
 adj_rhs_vjp adds the adjoint of the values H to hbar; the derivative being
 linear in it, one adj_hoist_vjp of the sum over all stages replaces the part of
-every stage's rhs_vjp that runs through them.
+every stage's rhs_vjp that runs through them.  These four run in FP32, where the
+roundings show: products that are added or subtracted are written as multiply-adds
+(cfg_fma), which rounds once, and alike in every kernel, where a compiler's
+contraction depends on what surrounds an expression.
 """
 from __future__ import annotations
 
@@ -85,8 +88,10 @@ def tissue_mode_body(stmts) -> List[Assign]:
 class _Gen:
     """Three-address forward code and the matching reverse sweep."""
 
-    def __init__(self, m: Model, early):
+    def __init__(self, m: Model, early, fused: bool = False):
         self.m = m
+        self.fused = fused
+        self.product: Dict[str, Tuple[str, str]] = {}   # value -> its factors
         self.early = set(early)
         self.params = {v: k for k, v in SCALABLE[m.name].items()}   # constant -> scale key
         self.n = 0
@@ -144,6 +149,20 @@ class _Gen:
             return self.cond(e, out, ind)
         return self.fwd(e, out, ind)
 
+    def binary(self, op: str, a: str, b: str, v: str) -> str:
+        if self.fused and op in "+-":
+            minus = "-" if op == "-" else ""
+            # of two products the left one, the larger where currents are added up
+            if a in self.product:
+                p, q = self.product[a]
+                return f"cfg_fma({p}, {q}, {minus}{b})"
+            if b in self.product:
+                p, q = self.product[b]
+                return f"cfg_fma({minus}{p}, {q}, {a})"
+        if op == "*":
+            self.product[v] = (a, b)
+        return f"({a} {op} {b})"
+
     def fwd(self, e: Node, out: List[str], ind: str) -> str:
         lf = self.leaf(e)
         if lf is not None:
@@ -175,7 +194,7 @@ class _Gen:
             a = self.fwd(e.l, out, ind)
             b = self.fwd(e.r, out, ind)
             v = self.tmp()
-            out.append(f"{ind}{v} = ({a} {e.op} {b});")
+            out.append(f"{ind}{v} = {self.binary(e.op, a, b, v)};")
             self.value[id(e)] = v
             return v
         if isinstance(e, Cond):
@@ -341,6 +360,8 @@ def _walk_body(gen: _Gen, body, fwd: List[str]):
             name = gen.tmp("a")
             fwd.append(f"    {name} = {v};")
             gen.defined[t.name] = name
+            if v in gen.product:
+                gen.product[name] = gen.product[v]
             gen.decl.append(f"    R b{name} = R(0);")
             targets.append((st, f"b{name}"))
         elif t.array == "RATES":
@@ -477,7 +498,7 @@ def emit_split(m: Model) -> str:
          f"__device__ __forceinline__ void adj_hoist(R y_{vm}, const KS& K, int tissue, R* H)",
          "{",
          "    (void)tissue;"]
-    gen = _Gen(m, [])
+    gen = _Gen(m, [], fused=True)
     fwd: List[str] = []
     targets = _walk_body(gen, first, fwd)
     L += gen.decl + fwd
@@ -491,7 +512,7 @@ def emit_split(m: Model) -> str:
           "{",
           "    (void)tissue;",
           f"    R ybar[1] = {{R(0)}};"]
-    gen = _Gen(m, [])
+    gen = _Gen(m, [], fused=True)
     fwd = []
     targets = _walk_body(gen, first, fwd)
     targets = [(st, n) for st, n in targets
@@ -499,7 +520,7 @@ def emit_split(m: Model) -> str:
     rev = [x.replace(f"ybar[S_{vm}]", "ybar[0]") for x in _reverse(gen, targets)]
     L += gen.decl + fwd + rev + ["    return ybar[0];", "}", ""]
 
-    gen = _Gen(m, use_before_def(m.rates))
+    gen = _Gen(m, use_before_def(m.rates), fused=True)
     gen.varying = {k for k, v in varying.items() if v}
     fwd = []
     targets = _walk_body(gen, rest, fwd)

@@ -76,6 +76,14 @@ CFG_HD __forceinline__ double cfg_fma(double a, double b, double c)
     return std::fma(a, b, c);
 #endif
 }
+CFG_HD __forceinline__ float cfg_fma(float a, float b, float c)
+{
+#ifdef __CUDA_ARCH__
+    return __fmaf_rn(a, b, c);
+#else
+    return std::fma(a, b, c);
+#endif
+}
 
 // a / b by the reciprocal r = RN(1 / b) at hand: the product, corrected once by
 // its exact remainder, which is the correctly rounded quotient but for rare
