@@ -205,10 +205,12 @@ __global__ void __launch_bounds__(kBlock) k_ionic_reverse(IonicArgs a)
 }
 
 // ------------------------------------------------------------------ mixed
-// The right-hand side and its derivative in FP32.  The stage sums, and the sums
-// of the adjoints over stages, are float pairs (48 bits, exact products) that
-// are rounded to FP32 only as inputs of the right-hand side; states and
-// adjoints are FP64 in memory and get the step's change added in FP64.
+// The right-hand side and its derivative in FP32, states and adjoints in FP64.
+// The change of a state over the step, and of the adjoints of states and
+// conductances, is summed in three floats (Acc3: more bits than FP64) and added
+// to FP64 memory at the end.  What goes into the right-hand side or its
+// derivative is a float, rounded once from a sum in float pairs (48 bits, exact
+// products) that starts from those values and is not carried further.
 //
 // What bounds these kernels is the instructions of a warp: 16,384 cells are one
 // warp for each of 512 of the chip's 608 SM partitions.  The FP64 sums they
@@ -242,7 +244,20 @@ struct CellConsts {
 struct PairTableau {
     fp::P a[7][6];              // h a_sj; row 6: h b_j
     double c[6];
+    // b_j over their common denominator, in whole numbers, and h over it
+    float whole_b[6];
+    fp::P unit;
+    double unit_d;
 };
+
+// 1/282150: the denominator of 16/135, 6656/12825, 28561/56430, -9/50 and 2/55
+constexpr double kWhole = 282150.0;
+constexpr double kWholeB[6] = {33440.0, 0.0, 146432.0, 142805.0, -50787.0, 10260.0};
+constexpr bool whole(double b, double n) { return b * kWhole - n < 1e-9 && n - b * kWhole < 1e-9; }
+static_assert(whole(rkf::b1, kWholeB[0]) && whole(rkf::b3, kWholeB[2]) &&
+                  whole(rkf::b4, kWholeB[3]) && whole(rkf::b5, kWholeB[4]) &&
+                  whole(rkf::b6, kWholeB[5]),
+              "the weights of the fifth-order solution");
 
 struct MixedArgs {
     IonicArgs a;
@@ -252,41 +267,51 @@ struct MixedArgs {
     float* ws;                  // [6 substeps + 1][NS - 1][threads] stage inputs (reverse)
 };
 
-// Adjoints are scaled by 2^kBarShift, so that the pairs' low parts of small ones
-// stay above FP32's smallest number.
-constexpr int kBarShift = 32;
-constexpr double kBarUnit = 1.0 / 4294967296.0;
-
-// One substep of (y, and its change dy since the start of the step); keep(s, Y)
-// is given the stage inputs.  The stages are a loop that is not unrolled, with
+// One substep; `sums` is the change of the state since y0, the start of the step,
+// in units of h / 282150: weighted with whole numbers the rates' products are exact
+// (y, the state itself, is formed anew at the substep's end).  keep(s, Y) is given
+// the stage inputs.  The stages are a loop that is not unrolled, with
 // the rates in shared memory (thread by thread, rows of a block's threads):
 // unrolled, the six right-hand sides are some 6000 instructions, and the one
 // warp of a partition waits for instructions half of the time (80 us for
-// 46 in the forward kernel).
+// 46 in the forward kernel, with sums of the state in pairs).
 using Rates = float[6][NS][kMixedBlock];
+
+// Sums in three floats, in shared memory beside the rates (registers are full of
+// what a stage needs).
+using Sums = float[NS][3][kMixedBlock];
+
+__device__ __forceinline__ fp::Acc3 load(const Sums& m, int i, int tid)
+{
+    fp::Acc3 a;
+    a.h = m[i][0][tid];
+    a.m = m[i][1][tid];
+    a.l = m[i][2][tid];
+    return a;
+}
+
+__device__ __forceinline__ void store(Sums& m, int i, int tid, const fp::Acc3& a)
+{
+    m[i][0][tid] = a.h;
+    m[i][1][tid] = a.m;
+    m[i][2][tid] = a.l;
+}
 
 template <class F>
 __device__ __forceinline__ void mixed_substep(const MixedArgs& g, double t, double h,
                                               const CellConsts& K, const float* H, Rates& k,
-                                              fp::P (&y)[NS], fp::P (&dy)[NS], F keep)
+                                              const double* y0, long long n,
+                                              fp::P (&y)[NS], Sums& sums, F keep)
 {
     const int tid = threadIdx.x;
 #pragma unroll 1
-    for (int s = 0; s <= 6; ++s) {       // 6: the substep's end
+    for (int s = 0; s < 6; ++s) {
         fp::Acc d[NS];
 #pragma unroll 1
         for (int j = 0; j < s; ++j) {
             const fp::P w = g.T.a[s][j];
 #pragma unroll
             for (int i = 1; i < NS; ++i) d[i].add_prod(w, k[j][i][tid]);
-        }
-        if (s == 6) {
-#pragma unroll
-            for (int i = 1; i < NS; ++i) {
-                y[i] = fp::add(y[i], d[i].value());
-                dy[i] = fp::add(dy[i], d[i].value());
-            }
-            break;
         }
         float Y[NS], ks[NS];
         Y[0] = y[0].x;
@@ -300,21 +325,36 @@ __device__ __forceinline__ void mixed_substep(const MixedArgs& g, double t, doub
 #pragma unroll
         for (int i = 1; i < NS; ++i) k[s][i][tid] = ks[i];
     }
+    fp::Acc3 dy[NS];
+#pragma unroll
+    for (int i = 1; i < NS; ++i) dy[i] = load(sums, i, tid);
+#pragma unroll 1
+    for (int j = 0; j < 6; j += j == 0 ? 2 : 1) {      // b_2 = 0
+        const float w = g.T.whole_b[j];
+#pragma unroll
+        for (int i = 1; i < NS; ++i) dy[i].add_prod(w, k[j][i][tid]);
+    }
+#pragma unroll
+    for (int i = 1; i < NS; ++i) {
+        store(sums, i, tid, dy[i]);
+        y[i] = fp::madd(g.T.unit, dy[i].value(), fp::split(y0[i * n]));
+    }
 }
 
-__device__ __forceinline__ void mixed_start(const double* y0, double vm, long long n, long long c,
-                                            fp::P (&y)[NS], fp::P (&dy)[NS])
+// the state at the start of the step; y0: of this cell, n apart
+__device__ __forceinline__ void mixed_start(const double* y0, double vm, long long n,
+                                            fp::P (&y)[NS], Sums& sums)
 {
     y[0] = fp::split(vm_to_state0<M::VM_MAP>(vm));
 #pragma unroll
     for (int i = 1; i < NS; ++i) {
-        y[i] = fp::split(y0[(long long)i * n + c]);
-        dy[i] = fp::make(0.0f);
+        y[i] = fp::split(y0[i * n]);
+        store(sums, i, threadIdx.x, fp::Acc3());
     }
 }
 
-// Forward ionic update of one PDE step: 254 us in FP64 sums, 46 us now
-// (16,384 cells, 5 substeps).
+// Forward ionic update of one PDE step: 254 us in FP64 sums, 52 us now
+// (16,384 cells, 5 substeps; 45 with the state's change in pairs, 48 bits).
 __global__ void __launch_bounds__(kMixedBlock) k_ionic_forward_mixed(
     const __grid_constant__ MixedArgs g)
 {
@@ -322,14 +362,15 @@ __global__ void __launch_bounds__(kMixedBlock) k_ionic_forward_mixed(
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= a.n) return;
     const CellConsts K(g.tissue, g.consts, a.n, c);
-    fp::P y[NS], dy[NS];
-    mixed_start(a.y, a.vm[c], a.n, c, y, dy);
+    __shared__ Rates k;
+    __shared__ Sums dy;
+    fp::P y[NS];
+    mixed_start(a.y + c, a.vm[c], a.n, y, dy);
     float H[tnnp::ADJ_NH];
     tnnp::adj_hoist<float>(y[0].x, K, g.a.tissue, H);
-    __shared__ Rates k;
     const double h = a.dtm / a.substeps;
     for (int j = 0; j < a.substeps; ++j)
-        mixed_substep(g, a.t0 + j * h, h, K, H, k, y, dy, [](int, const float*) {});
+        mixed_substep(g, a.t0 + j * h, h, K, H, k, a.y + c, a.n, y, dy, [](int, const float*) {});
     float yr[NS], d[NS];
 #pragma unroll
     for (int i = 0; i < NS; ++i) yr[i] = y[i].x;
@@ -337,7 +378,7 @@ __global__ void __launch_bounds__(kMixedBlock) k_ionic_forward_mixed(
     a.im[c] = double(iion) * M::IION_SCALE;
     a.y[c] = vm_to_state0<M::VM_MAP>(a.vm[c]);
 #pragma unroll
-    for (int i = 1; i < NS; ++i) a.y[(long long)i * a.n + c] += fp::join(dy[i]);
+    for (int i = 1; i < NS; ++i) a.y[(long long)i * a.n + c] += load(dy, i, threadIdx.x).join() * g.T.unit_d;
 }
 
 // Reverse of one PDE step of the ionic update: the forward pass again, keeping
@@ -345,7 +386,7 @@ __global__ void __launch_bounds__(kMixedBlock) k_ionic_forward_mixed(
 // backwards.  With yb the adjoint of a substep's end and Yb_s that of the stage
 // inputs, the adjoint of rate s is h b_s yb + sum_{l > s} h a_ls Yb_l, and that
 // of the substep's start yb + sum_s Yb_s.  989 us in FP64 sums with the stages
-// formed twice, 119 us now (16,384 cells, 5 substeps).
+// formed twice, 159 us now (16,384 cells, 5 substeps; 119 with all sums in pairs).
 __global__ void __launch_bounds__(kMixedBlock) k_ionic_reverse_mixed(
     const __grid_constant__ MixedArgs g)
 {
@@ -355,28 +396,35 @@ __global__ void __launch_bounds__(kMixedBlock) k_ionic_reverse_mixed(
     const double h = a.dtm / a.substeps;
     const int last = 6 * a.substeps, tid = threadIdx.x;
     __shared__ Rates yk;                 // forward: the rates; backward: Yb
+    __shared__ Sums sums;                // change of the state; of its adjoint
     for (long long c = slot; c < a.n; c += slots) {
         const CellConsts K(g.tissue, g.consts, a.n, c);
         float H[tnnp::ADJ_NH], V;
         {
-            fp::P y[NS], dy[NS];
-            mixed_start(a.y_start, a.vm[c], a.n, c, y, dy);
+            fp::P y[NS];
+            const double* y0 = a.y_start + c;
+            mixed_start(y0, a.vm[c], a.n, y, sums);
             V = y[0].x;
             tnnp::adj_hoist<float>(V, K, g.a.tissue, H);
             float* w = g.ws + slot;
             for (int j = 0; j < a.substeps; ++j)
-                mixed_substep(g, a.t0 + j * h, h, K, H, yk, y, dy, [&](int, const float* Y) {
+                mixed_substep(g, a.t0 + j * h, h, K, H, yk, y0, a.n, y, sums, [&](int, const float* Y) {
 #pragma unroll
                     for (int i = 1; i < NS; ++i, w += slots) *w = Y[i];
                 });
 #pragma unroll
             for (int i = 1; i < NS; ++i, w += slots) *w = y[i].x;
         }
+        // adjoints enter scaled by 2^32, so that the low parts of small ones stay
+        // above FP32's smallest number
+        constexpr int shift = 32;
+        constexpr double unit = 1.0 / 4294967296.0;
+        const double* yb0 = a.ybar + c;
+        const double ib = a.imbar[c] * M::IION_SCALE;
         fp::P yb[NS];
-        fp::Acc dyb[NS], hb[tnnp::ADJ_NH], pb[6];
+        fp::Acc3 vb, hb[tnnp::ADJ_NH], pb[6];
 #pragma unroll
-        for (int i = 1; i < NS; ++i)
-            yb[i] = fp::split(a.ybar[(long long)i * a.n + c], kBarShift);
+        for (int i = 1; i < NS; ++i) store(sums, i, tid, fp::Acc3());
         int s = 0;
 #pragma unroll 1
         for (int it = last; it >= 0; --it) {
@@ -398,7 +446,7 @@ __global__ void __launch_bounds__(kMixedBlock) k_ionic_reverse_mixed(
             const bool end = it == last;
             float ibar = 0.0f;
             if (end) {
-                ibar = fp::split(a.imbar[c] * M::IION_SCALE, kBarShift).x;
+                ibar = fp::split(ib, shift).x;
             } else {
                 fp::Acc d[NS];
                 const fp::P b = g.T.a[6][s];
@@ -414,39 +462,41 @@ __global__ void __launch_bounds__(kMixedBlock) k_ionic_reverse_mixed(
                 for (int i = 1; i < NS; ++i) dbar[i] = __fadd_rn(d[i].h, d[i].l);
             }
             tnnp::adj_rhs_vjp<float>(0.0, Y, K, g.a.tissue, H, dbar, ibar, Ys, pbar, hbar);
-            dyb[0].add(Ys[0]);
+            vb.add(Ys[0]);
 #pragma unroll
             for (int q = 0; q < tnnp::ADJ_NH; ++q) hb[q].add(hbar[q]);
 #pragma unroll
             for (int q = 0; q < 6; ++q) pb[q].add(pbar[q]);
 #pragma unroll
-            for (int i = 1; i < NS; ++i) {
-                dyb[i].add(Ys[i]);
-                yk[s][i][tid] = Ys[i];
-            }
+            for (int i = 1; i < NS; ++i) yk[s][i][tid] = Ys[i];
             if (s == 0) {            // the end of the step, or a substep's start
-                fp::Acc d[NS];
+                fp::Acc3 d[NS];
+#pragma unroll
+                for (int i = 1; i < NS; ++i) d[i] = load(sums, i, tid);
 #pragma unroll 1
                 for (int l = end ? 0 : 5; l >= 0; --l)
 #pragma unroll
                     for (int i = 1; i < NS; ++i) d[i].add(yk[l][i][tid]);
 #pragma unroll
-                for (int i = 1; i < NS; ++i) yb[i] = fp::add(yb[i], d[i].value());
+                for (int i = 1; i < NS; ++i) {
+                    store(sums, i, tid, d[i]);
+                    yb[i] = fp::add(fp::split(yb0[i * a.n], shift), d[i].value());
+                }
             }
             s = s == 0 ? 5 : s - 1;
         }
-        float hbar[tnnp::ADJ_NH];
+        float hbar[tnnp::ADJ_NH];    // rounded once here, where every stage's would be
 #pragma unroll
         for (int q = 0; q < tnnp::ADJ_NH; ++q) hbar[q] = hb[q].value().x;
-        dyb[0].add(tnnp::adj_hoist_vjp<float>(V, K, g.a.tissue, hbar));
-        a.vbar[c] += fp::join(dyb[0].value()) * (kBarUnit * vm_map_slope<M::VM_MAP>());
+        vb.add(tnnp::adj_hoist_vjp<float>(V, K, g.a.tissue, hbar));
+        a.vbar[c] += vb.join() * (unit * vm_map_slope<M::VM_MAP>());
         a.ybar[c] = 0.0;
 #pragma unroll
         for (int i = 1; i < NS; ++i)
-            a.ybar[(long long)i * a.n + c] += fp::join(dyb[i].value()) * kBarUnit;
+            a.ybar[(long long)i * a.n + c] += load(sums, i, tid).join() * unit;
 #pragma unroll
         for (int q = 0; q < 6; ++q)
-            a.pbar[(long long)q * a.n + c] += fp::join(pb[q].value()) * kBarUnit;
+            a.pbar[(long long)q * a.n + c] += pb[q].join() * unit;
     }
 }
 
@@ -816,8 +866,11 @@ MixedArgs mixed_args(cfg_adjoint* a, const IonicArgs& g)
     for (int s = 0; s < 6; ++s) {
         for (int j = 0; j < 5; ++j) m.T.a[s][j] = pair(h * ra[s][j]);
         m.T.a[6][s] = pair(h * rb[s]);
+        m.T.whole_b[s] = float(kWholeB[s]);
         m.T.c[s] = rc[s];
     }
+    m.T.unit_d = h / kWhole;
+    m.T.unit = pair(m.T.unit_d);
     double C[M::NC] = {}, y[NS] = {};
     M::init(C, y, a->tissue, nullptr);
     for (int i = 0; i < M::NC; ++i) m.tissue[i] = float(C[i]);

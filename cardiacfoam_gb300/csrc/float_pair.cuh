@@ -118,6 +118,30 @@ struct Acc {
     __device__ __forceinline__ P value() const { return quick(h, l); }
 };
 
+// Sum of floats, and of products of two floats, in three floats: each holds the
+// rounding errors of the one before, so the sum carries more bits than FP64 does,
+// for 13 and 22 operations of the FP32 pipe.
+struct Acc3 {
+    float h = 0.0f, m = 0.0f, l = 0.0f;
+    __device__ __forceinline__ void add(float b)
+    {
+        const P s = two_sum(h, b), t = two_sum(m, s.y);
+        h = s.x;
+        m = t.x;
+        l = __fadd_rn(l, t.y);
+    }
+    __device__ __forceinline__ void add_prod(float a, float b)
+    {
+        const float p = __fmul_rn(a, b), e = __fmaf_rn(a, b, -p);
+        const P s = two_sum(h, p), t = two_sum(m, s.y), u = two_sum(t.x, e);
+        h = s.x;
+        m = u.x;
+        l = __fadd_rn(l, __fadd_rn(t.y, u.y));
+    }
+    __device__ __forceinline__ P value() const { return quick(h, m); }   // its leading pair
+    __device__ __forceinline__ double join() const { return double(h) + (double(m) + double(l)); }
+};
+
 // v * 2^shift as a renormalised pair, from the bit pattern of v with integer
 // operations (the FP64 pipe is not used): hi takes the leading 24
 // significant bits (truncated), lo the next 29 rounded to 24, which leaves

@@ -435,7 +435,9 @@ typedef struct cfg_adjoint_desc {
     int pcg_max_iter;
     int precision;               /* CFG_PRECISION_FP64, or _MIXED: the ionic right-hand
                                     side and its derivative in FP32, states and
-                                    adjoint accumulations in FP64 */
+                                    adjoints in FP64; their changes over a step
+                                    are summed in three floats, which hold more
+                                    bits than FP64 */
 } cfg_adjoint_desc;
 
 typedef struct cfg_adjoint cfg_adjoint;
