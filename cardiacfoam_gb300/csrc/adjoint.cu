@@ -341,6 +341,12 @@ __device__ __forceinline__ void mixed_substep(const MixedArgs& g, double t, doub
     }
 }
 
+// binary exponent of v from its bits
+__device__ __forceinline__ int exponent(double v)
+{
+    return ((__double2hiint(v) >> 20) & 0x7ff) - 1023;
+}
+
 // the state at the start of the step; y0: of this cell, n apart
 __device__ __forceinline__ void mixed_start(const double* y0, double vm, long long n,
                                             fp::P (&y)[NS], Sums& sums)
@@ -415,12 +421,16 @@ __global__ void __launch_bounds__(kMixedBlock) k_ionic_reverse_mixed(
 #pragma unroll
             for (int i = 1; i < NS; ++i, w += slots) *w = y[i].x;
         }
-        // adjoints enter scaled by 2^32, so that the low parts of small ones stay
-        // above FP32's smallest number
-        constexpr int shift = 32;
-        constexpr double unit = 1.0 / 4294967296.0;
+        // adjoints enter scaled by a power of two: 2^32, so that the low parts of
+        // small ones stay above FP32's smallest number, or less where the largest
+        // would leave 2^60
         const double* yb0 = a.ybar + c;
         const double ib = a.imbar[c] * M::IION_SCALE;
+        int top = exponent(ib);
+#pragma unroll
+        for (int i = 1; i < NS; ++i) top = max(top, exponent(yb0[i * a.n]));
+        const int shift = min(32, 60 - top);
+        const double unit = __hiloint2double((1023 - shift) << 20, 0);
         fp::P yb[NS];
         fp::Acc3 vb, hb[tnnp::ADJ_NH], pb[6];
 #pragma unroll
