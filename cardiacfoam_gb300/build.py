@@ -25,8 +25,8 @@ INCLUDE = PKG.parent / "include"
 
 MODELS = ["tnnp", "ord", "torord_dyncl", "alievpanfilov", "buenoorovio",
           "monodomainfdamanufactured", "bidomainfdamanufactured"]
-# per-model unroll factor of the per-state loops around the right-hand side
-# (measured on GB300: ORd fastest at 4, the others at 1)
+# per-model unroll factor of the FP64 batch's loops over the states (10 steps of
+# ORd: 30,000 cells 27.0 ms at 4 and 28.7 at 1, 4,800 cells 14.0 and 13.2)
 STATE_UNROLL = {"ord": 4}
 # resident blocks of 64 per SM the mixed kernel is built for, where the
 # model's registers (right-hand side plus the state held in registers) and

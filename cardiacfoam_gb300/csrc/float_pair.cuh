@@ -167,17 +167,5 @@ __device__ __forceinline__ P split(double v, int shift = 0)
     return quick(hi, __uint_as_float(__float_as_uint(rem) | sign));
 }
 
-// Warp sum of pairs in a fixed tree (lane 0 holds the result)
-__device__ __forceinline__ P warp_sum(P v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const P w = make_float2(__shfl_down_sync(0xffffffffu, v.x, o),
-                                __shfl_down_sync(0xffffffffu, v.y, o));
-        v = add(v, w);
-    }
-    return v;
-}
-
 }  // namespace fp
 }  // namespace cfg

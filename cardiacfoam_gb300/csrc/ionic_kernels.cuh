@@ -27,9 +27,9 @@
 #ifndef CFG_IONIC_MIN_BLOCKS
 #define CFG_IONIC_MIN_BLOCKS 2
 #endif
-// unroll factor of the per-state loops around the right-hand side (stage
-// sums, 5th-order update, error norm); 1 keeps the kernel's instruction
-// footprint close to one copy of the model body
+// unroll factor of the FP64 batch's loops over the states (stage sums,
+// 5th-order update, error norm); 1 keeps the kernel's instruction footprint
+// close to one copy of the model body
 #ifndef CFG_IONIC_STATE_UNROLL
 #define CFG_IONIC_STATE_UNROLL 1
 #endif

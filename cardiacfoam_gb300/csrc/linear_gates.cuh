@@ -56,7 +56,6 @@ static_assert(small(kPolys.e[0]) && small(kPolys.e[1]) && small(kPolys.e[2]) &&
                   small(kPolys.e[3]),
               "the embedded pair's error starts at z^4");
 
-CFG_D __forceinline__ float fma_r(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 CFG_D __forceinline__ double fma_r(double a, double b, double c) { return __fma_rn(a, b, c); }
 
 // single coefficients as scalar constants (device code cannot index kPolys)
@@ -91,27 +90,12 @@ CFG_D __forceinline__ R error_poly(R z)
 
 }  // namespace lingate
 
-// Split of a model's states in tissue mode: state 0 (Vm) does not change,
-// the linear gates follow the polynomials above, the rest goes through the
-// stage slots.  nl(i) / g(i): index of state i among the rest / the gates.
+// The linear gates among a model's states in tissue mode: they follow the
+// polynomials above.  State 0 (Vm) does not change, the others go through the
+// stage slots.
 template <class M>
 struct TissueSplit {
     static CFG_HD constexpr bool lin(int i) { return i > 0 && ((M::LIN_MASK >> i) & 1ull); }
-    static CFG_HD constexpr bool rest(int i) { return i > 0 && !lin(i); }
-    static CFG_HD constexpr int g(int i)
-    {
-        int k = 0;
-        for (int j = 1; j < i; ++j) k += lin(j) ? 1 : 0;
-        return k;
-    }
-    static CFG_HD constexpr int nl(int i)
-    {
-        int k = 0;
-        for (int j = 1; j < i; ++j) k += rest(j) ? 1 : 0;
-        return k;
-    }
-    static constexpr int NL = nl(M::NS), NG = g(M::NS);
-    static constexpr int NLA = NL > 0 ? NL : 1, NGA = NG > 0 ? NG : 1;
 };
 
 }  // namespace cfg
