@@ -22,10 +22,11 @@
 // and z in one pass, where each had a pass and a barrier; and a corrector
 // whose predecessor needed no iteration and had the same right-hand side is
 // that predecessor again (same x, same b), so its recorded result is repeated.
-// Measured per step, before and after all of this (steady state, 3 + 0 + 0
-// iterations): 3,360 cells in FP64 96 to 46 us, 52,500 in FP64 114 to 69 us,
-// 420,000 in float pairs 133 to 111 us, the 563,921-cell ventricle in float
-// pairs 384 to 305 us.
+// Measured per step, before and after all of this: 3,360 cells in FP64 95 to
+// 46 us, 52,500 in FP64 114 to 72 us, 420,000 in float pairs 133 to 111 us
+// (steady state, 3 + 0 + 0 iterations), a ventricle of 563,616 tetrahedra with its
+// corrections 379 to 301 us in FP64, the default there, and 299 to 265 in float
+// pairs.
 //
 // On a general mesh every corrector first forms the cell gradient of the
 // iterate (one more barrier) for the explicit correction of the Laplacian

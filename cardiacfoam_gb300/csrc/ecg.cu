@@ -125,9 +125,9 @@ __device__ __forceinline__ void finish(const EcgArgs& a, const Acc<PAIR> (&acc)[
                                        double (*red)[kEcgBlock], bool& last)
 {
     // a warp per electrode adds the threads' values: a shuffle tree per electrode in
-    // every warp takes four times as many FP64 additions, of 64 clocks each (an
-    // evaluation of 563,616 cells at five electrodes 15.8 us with them, 13.3 so; at
-    // 83,520 cells it is 10 us, the launch and the wait for the last block)
+    // every warp takes four times as many FP64 additions, of 64 clocks each (32
+    // evaluations of 563,616 cells at five electrodes 502 us with them, 468 so;
+    // back to back 14.4 and 13.2 us each, near what the host takes to issue one)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int j = 0; j < NE; ++j) red[j][threadIdx.x] = acc[j].value();
