@@ -198,22 +198,25 @@ __global__ void __launch_bounds__(128) batch_fp64_kernel(BatchLaunch p)
     }
 }
 
-// Mixed form: FP32 arithmetic, slow states as (hi, lo) pairs, the state and the
-// stage data in shared memory (see ionic_mixed.cuh).
+// Mixed form: FP32 arithmetic, slow states as (hi, lo) pairs, the stage data in
+// shared memory (see ionic_mixed.cuh), the first R states in registers and the
+// others in shared memory too.
 //
-// What bounds it is the fetch of instructions: with a warp or two on an SM
-// partition nothing hides it, and the loops over the states, unrolled for a state
-// in registers, are as long as the right-hand side (half of a warp's time went to
-// it for 16,384 ToRORd cells).  With the state in shared memory they are loops.
-// 300 steps of those cells take 34.4 ms instead of 55.1, 100 steps of 65,536 cells
-// 74.9 instead of 91.9 (TNNP 37.9 for 43.1).  Up to a warp per SM the registers'
-// form is 1 % (TNNP) to 3 % (ORd) faster, and 1 to 8 % slower in the other models;
-// it rounds otherwise in places, and a cell's result must not depend on how many
-// others there are, so every population takes this form.
-template <class M>
-struct BatchSlice {
+// What bounds it is the fetch of instructions while a warp or two on an SM partition
+// cannot hide it: loops over the states that are unrolled, as registers need, are as
+// long as the right-hand side (half of a warp's time for 16,384 ToRORd cells).  With
+// more cells it is the warps that fit an SM, which states in shared memory cost.  So
+// all states are in memory while every cell is resident that way, and beyond that as
+// few in registers as leave the warps that registers alone would (19 of ToRORd's 45,
+// 26 of ORd's 41).  Both forms, and all states in registers, give the same bits.
+// ToRORd, all in registers / all in memory / 19 in registers: 1200 steps of 16,384
+// cells 102 / 74 / 80 ms, their upstroke (300 steps) 55 / 30 / 38; 1200 steps of
+// 32,768 cells 106 / 146 / 91; 2000 steps of 65,536 cells 260 / 283 / 226.
+template <class M, int R>
+struct BatchShape {
     using S = mixed::Slice<M>;
-    static constexpr int len = (S::raw + S::NSP + S::NW) | 1;   // stages, Y, LO
+    using State = mixed::CellState<M, R>;
+    static constexpr int len = (S::raw + M::NS - R + S::NW - State::RW) | 1;   // stages, state
     static constexpr int block =
         32 * mixed::blocks_per_sm(32, len) > 64 * mixed::blocks_per_sm(64, len) ? 32 : 64;
     static constexpr int fit = mixed::blocks_per_sm(block, len);
@@ -224,19 +227,28 @@ struct BatchSlice {
 #endif
     static constexpr int min_blocks = want < 1 ? 1 : (want > 16 ? 16 : want);
     static constexpr int smem_bytes = block * len * 4;
+    static constexpr int threads = block * min_blocks;   // per SM
 };
 
-template <class M, int T>
-__global__ void __launch_bounds__(BatchSlice<M>::block, BatchSlice<M>::min_blocks)
+// states in registers of a population that is not resident at once
+template <class M, int R = 0>
+constexpr int batch_registers()
+{
+    if constexpr (BatchShape<M, R>::threads >= BatchShape<M, M::NS>::threads) return R;
+    else return batch_registers<M, R + 1>();
+}
+
+template <class M, int T, int R>
+__global__ void __launch_bounds__(BatchShape<M, R>::block, BatchShape<M, R>::min_blocks)
 batch_mixed_kernel(BatchLaunch p)
 {
     using S = mixed::Slice<M>;
     using L = Layout<M, false>;
-    constexpr int NS = M::NS, P = S::NSP, U = 4;
+    constexpr int NS = M::NS, P = S::NSP;
     extern __shared__ float cfg_batch_smem[];
-    float* K = cfg_batch_smem + threadIdx.x * BatchSlice<M>::len;
-    float* Y = K + S::raw;
-    float* LO = Y + S::NSP;
+    float* K = cfg_batch_smem + threadIdx.x * BatchShape<M, R>::len;
+    mixed::CellState<M, R> Y;
+    Y.mem = K + S::raw;
     unsigned evals = 0;
     for (;;) {
         const long long c = (long long)atomicAdd(p.queue, 1ull);
@@ -251,10 +263,10 @@ batch_mixed_kernel(BatchLaunch p)
         for (int i = 0; i < NS; ++i) {
             if (is_wide<M::WIDE_MASK>(i)) {
                 const float2 v = yw2[(long long)L::slot(i) * p.n + c];
-                Y[i] = v.x;
-                LO[w++] = v.y;
+                Y.at(i) = v.x;
+                Y.low_at(w++) = v.y;
             } else {
-                Y[i] = p.yn[(long long)L::slot(i) * p.n + c];
+                Y.at(i) = p.yn[(long long)L::slot(i) * p.n + c];
             }
         }
         float dep[M::NSD > 0 ? M::NSD : 1];
@@ -274,24 +286,23 @@ batch_mixed_kernel(BatchLaunch p)
             dx_try = fminf(dx_try, float(dtm));
             IonicFailure why;
             float iion;
-            const long long nsub = mixed::solve<M, true, U>(ts, te, float(dtm), Y, K, LO,
-                                                         dx_try, Kc, T, stim, p.ode, evals,
-                                                         why, iion);
+            const long long nsub = mixed::solve<M, true>(ts, te, float(dtm), Y, K, dx_try, Kc, T,
+                                                         stim, p.ode, evals, why, iion);
             if (nsub < 0) {
                 batch_fail(p, c, why);
                 failed = true;
                 break;
             }
             t = t_new;
-            const double v0 = is_wide<M::WIDE_MASK>(0) ? double(Y[0]) + double(LO[0])
-                                                       : double(Y[0]);
+            const double v0 = is_wide<M::WIDE_MASK>(0) ? double(Y.at(0)) + double(Y.low_at(0))
+                                                       : double(Y.at(0));
             double ca = 0.0;
             if constexpr (M::CA_STATE >= 0) {
                 if (is_wide<M::WIDE_MASK>(M::CA_STATE)) {
                     constexpr int wc = Layout<M, false>::slot(M::CA_STATE);
-                    ca = double(Y[M::CA_STATE]) + double(LO[wc]);
+                    ca = double(Y.at(M::CA_STATE)) + double(Y.low_at(wc));
                 } else {
-                    ca = double(Y[M::CA_STATE]);
+                    ca = double(Y.at(M::CA_STATE));
                 }
             }
             batch_sample<M>(p, c, k + 1, a, t, v0, ca);
@@ -301,9 +312,9 @@ batch_mixed_kernel(BatchLaunch p)
 #pragma unroll
         for (int i = 0; i < NS; ++i) {
             if (is_wide<M::WIDE_MASK>(i))
-                yw2o[(long long)L::slot(i) * p.n + c] = make_float2(Y[i], LO[w++]);
+                yw2o[(long long)L::slot(i) * p.n + c] = make_float2(Y.at(i), Y.low_at(w++));
             else
-                p.yn[(long long)L::slot(i) * p.n + c] = Y[i];
+                p.yn[(long long)L::slot(i) * p.n + c] = Y.at(i);
         }
         p.step[c] = double(dx_try);
         p.t[c] = t;

@@ -167,27 +167,12 @@ extern "C" void CFG_CAT3(cfg_ionic_host_init_, CFG_MODEL, )(double* C, double* y
 
 // ---------------------------------------------------------------- batched single cells
 
-template <int T>
-static cudaError_t batch_launch(const cfg::BatchLaunch& p, cudaStream_t s)
+// persistent grid: every block resident, cells handed out by the queue
+static cudaError_t batch_launch_on(void (*fn)(cfg::BatchLaunch), int& per_sm, int sms, int block,
+                                   int smem, const cfg::BatchLaunch& p, cudaStream_t s)
 {
-    int block, smem;
-    void (*fn)(cfg::BatchLaunch);
-    if constexpr (kFP64) {
-        fn = cfg::batch_fp64_kernel<M, T>;
-        block = 128;
-        smem = 0;
-    } else {
-        fn = cfg::batch_mixed_kernel<M, T>;
-        block = cfg::BatchSlice<M>::block;
-        smem = cfg::BatchSlice<M>::smem_bytes;
-    }
-    // persistent grid: every block resident, cells handed out by the queue
-    static int per_sm = 0, sms = 0;
     if (!per_sm) {
-        int dev = 0;
-        cudaError_t e = cudaGetDevice(&dev);
-        if (!e) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (!e) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, block, smem);
+        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, block, smem);
         if (e) return e;
         if (per_sm < 1) per_sm = 1;
     }
@@ -196,6 +181,35 @@ static cudaError_t batch_launch(const cfg::BatchLaunch& p, cudaStream_t s)
     const unsigned grid = unsigned(want < cap ? want : cap);
     fn<<<grid, block, smem, s>>>(p);
     return cudaGetLastError();
+}
+
+template <int T>
+static cudaError_t batch_launch(const cfg::BatchLaunch& p, cudaStream_t s)
+{
+    static int sms = 0, per_sm = 0;
+    if (!sms) {
+        int dev = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (!e) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (e) return e;
+    }
+    if constexpr (kFP64) {
+        return batch_launch_on(cfg::batch_fp64_kernel<M, T>, per_sm, sms, 128, 0, p, s);
+    } else {
+        // all states in shared memory while every cell is resident that way; see
+        // ionic_batch.cuh for both sides
+        using All = cfg::BatchShape<M, 0>;
+        constexpr int R = cfg::batch_registers<M>();
+        if constexpr (R > 0) {
+            using Some = cfg::BatchShape<M, R>;
+            static int per_sm_some = 0;
+            if (p.n > (long long)sms * All::threads)
+                return batch_launch_on(cfg::batch_mixed_kernel<M, T, R>, per_sm_some, sms,
+                                       Some::block, Some::smem_bytes, p, s);
+        }
+        return batch_launch_on(cfg::batch_mixed_kernel<M, T, 0>, per_sm, sms, All::block,
+                               All::smem_bytes, p, s);
+    }
 }
 
 template <int T0, int... TR>
@@ -207,27 +221,27 @@ static cudaError_t batch_dispatch(const cfg::BatchLaunch& p, int tissue, cudaStr
     return cudaErrorInvalidValue;
 }
 
-template <int... TS>
+template <int R, int... TS>
 static cudaError_t batch_prepare(TissueList<TS...>)
 {
-    if constexpr (kFP64) {
-        return cudaSuccess;
-    } else {
+    if constexpr (!kFP64) {
         cudaError_t r[] = {cudaSuccess,
-                           cudaFuncSetAttribute(&cfg::batch_mixed_kernel<M, TS>,
+                           cudaFuncSetAttribute(&cfg::batch_mixed_kernel<M, TS, R>,
                                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                cfg::BatchSlice<M>::smem_bytes)...};
+                                                cfg::BatchShape<M, R>::smem_bytes)...};
         for (cudaError_t x : r)
             if (x) return x;
-        return cudaSuccess;
     }
+    return cudaSuccess;
 }
 
 extern "C" cudaError_t CFG_CAT3(cfg_batch_init_, CFG_MODEL, CFG_PREC_TAG)(
     const cfg::BatchLaunch& p, const double* scales, int tissue, double init_step,
     cudaStream_t stream)
 {
-    if (cudaError_t e = batch_prepare(Tissues{})) return e;
+    if (cudaError_t e = batch_prepare<0>(Tissues{})) return e;
+    if constexpr (cfg::batch_registers<M>() > 0)
+        if (cudaError_t e = batch_prepare<cfg::batch_registers<M>()>(Tissues{})) return e;
     if (p.n <= 0) return cudaSuccess;
     const int block = 128;
     const unsigned grid = unsigned((p.n + block - 1) / block);

@@ -5,12 +5,13 @@
 // overflow the L1 at useful occupancy and round-trip through L2/DRAM.  Here
 // each thread owns a slice of dynamic shared memory instead:
 //
-//   Y[NSP]   states in FP32 (the high part for the slow states)
-//   T[NSP]   stage input
-//   K[5][NSP] stage slots: k1..k5, then (after the stage-6 input is formed)
+//   K[5][NSP] stage slots: k1..k5 (a stage's input stands in the slot its
+//            derivative goes to), then (after the stage-6 input is formed)
 //            P = sum b_j k_j (j<6), E = sum e_j k_j (j<6), k6, and the FP32
 //            round-off bound of E
-//   LO[NW]   low parts of the slow (WIDE_MASK) states
+//   the states that are not in registers, and the low parts of the slow
+//   (WIDE_MASK) ones among them (CellState: tissue kernels keep all states in
+//   registers, batches all or some in the slice)
 //
 // The slice length is odd, so the 32 threads of a warp touching the same
 // element hit 32 different banks.
@@ -43,8 +44,7 @@ constexpr int blocks_per_sm(int block, int len)
     return kSmemPerSm / (block * len * 4 + kSmemReserve);
 }
 
-// Per thread: the five stage slots in shared memory (the state Y and the
-// low parts of the slow states live in registers).
+// Per thread: the five stage slots in shared memory, with all states in registers.
 template <class M>
 struct Slice {
     static constexpr int NSP = M::NS | 1;   // odd stride for each array
@@ -102,14 +102,8 @@ CFG_D __forceinline__ void add_wide(float& hi, float& lo, float d)
     hi = h;
 }
 
-// The accepted state from a loop that is not unrolled.  Unrolled, the compiler
-// shares the error norm's y5 = fma(h, q, y0) and rounded increment with the update;
-// the same values here keep the roundings of both forms alike.
-CFG_D __forceinline__ float accept_narrow(float y, float h, float q)
-{
-    return __fmaf_rn(h, q, y);
-}
-
+// hi + lo += h q, as the sum of a state's update rounds: fma(h, q, hi) and the
+// rounded increment
 CFG_D __forceinline__ void accept_wide(float& hi, float& lo, float h, float q)
 {
     const float s = __fmaf_rn(h, q, hi), d = __fmul_rn(h, q);
@@ -120,47 +114,118 @@ CFG_D __forceinline__ void accept_wide(float& hi, float& lo, float h, float q)
     lo = __fsub_rn(l, __fsub_rn(hi, s));
 }
 
+// a b + c d, and a b + c
+CFG_D __forceinline__ float mul2(float a, float b, float c, float d)
+{
+    return __fmaf_rn(a, b, __fmul_rn(c, d));
+}
+CFG_D __forceinline__ float mad(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+
+// A cell's state and the low parts of its slow states: the first R states in
+// registers, which takes loops that are unrolled, the others in memory, which
+// leaves them loops.  With states in memory (kExact) every rounding is written out:
+// as the compiler chooses them for the unrolled form, which leaves a product that is
+// used by itself too out of a multiply-add, so that a cell's result does not depend
+// on R.
+template <class M, int R_>
+struct CellState {
+    static constexpr int NS = M::NS, R = R_;
+    static constexpr bool kExact = R < NS;
+    static constexpr int wide_before(int n)
+    {
+        int k = 0;
+        for (int i = 0; i < n; ++i) k += is_wide<M::WIDE_MASK>(i) ? 1 : 0;
+        return k;
+    }
+    static constexpr int RW = wide_before(R);
+    float reg[R > 0 ? R : 1];
+    float low[RW > 0 ? RW : 1];
+    float* mem;          // [NS - R], then the low parts of the slow ones among them
+
+    // state i and the low part of slow state number w, i and w constants
+    CFG_D __forceinline__ float& at(int i) { return i < R ? reg[i] : mem[i - R]; }
+    CFG_D __forceinline__ float& low_at(int w) { return w < RW ? low[w] : mem[NS - R + w - RW]; }
+    // f(i, state i, low part of state i if it is a slow one) for every state
+    template <class F>
+    CFG_D __forceinline__ void each(F f)
+    {
+        int w = 0;
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            f(i, reg[i], low[w < RW ? w : 0]);
+            if (is_wide<M::WIDE_MASK>(i)) ++w;
+        }
+        if constexpr (R < NS) {
+            float* lo = mem + NS - R;
+#pragma unroll 4
+            for (int i = R; i < NS; ++i) {
+                f(i, mem[i - R], *lo);
+                if (is_wide<M::WIDE_MASK>(i)) ++lo;
+            }
+        }
+    }
+    // state i at a run-time index (for failure records)
+    CFG_D __forceinline__ double value(int i) const
+    {
+        float v = 0.0f;
+#pragma unroll
+        for (int k = 0; k < R; ++k)
+            if (k == i) v = reg[k];
+        if (R < NS && i >= R) v = mem[i - R];
+        return double(v);
+    }
+};
+
 // Stage input T = Y + h * sum_j a_sj k_j for stages 2..5 (s = 1..4); T is
 // the stage's own slot K + s P, where its derivative is then evaluated in
 // place.
-// Y is an array of registers, with loops unrolled all the way (U = NS), or a
-// pointer, with any U.  (The stage-6 sums stay unrolled: as a loop they gain 12 %
-// but the compiler fuses their products otherwise.)
-template <class M, int U, class YT>
-CFG_D __forceinline__ void stage_input(int s, float h, const YT& Y, float* T, const float* K)
+template <class M, class ST>
+CFG_D __forceinline__ void stage_input(int s, float h, ST& Y, float* T, const float* K)
 {
-    constexpr int NS = M::NS, P = Slice<M>::NSP;
+    constexpr int P = Slice<M>::NSP;
     switch (s) {
     case 1:
-#pragma unroll U
-        for (int i = 0; i < NS; ++i) T[i] = Y[i] + h * (fa21 * K[i]);
+        Y.each([&](int i, float y, float) {
+            if constexpr (ST::kExact) T[i] = mad(h, __fmul_rn(fa21, K[i]), y);
+            else T[i] = y + h * (fa21 * K[i]);
+        });
         break;
     case 2:
-#pragma unroll U
-        for (int i = 0; i < NS; ++i) {
+        Y.each([&](int i, float y, float) {
+            if constexpr (ST::kExact) {
+                T[i] = mad(h, mul2(fa31, K[i], fa32, K[P + i]), y);
+                return;
+            }
             float acc = fa31 * K[i];
             acc += fa32 * K[P + i];
-            T[i] = Y[i] + h * acc;
-        }
+            T[i] = y + h * acc;
+        });
         break;
     case 3:
-#pragma unroll U
-        for (int i = 0; i < NS; ++i) {
+        Y.each([&](int i, float y, float) {
+            if constexpr (ST::kExact) {
+                T[i] = mad(h, mad(fa43, K[2 * P + i], mul2(fa41, K[i], fa42, K[P + i])), y);
+                return;
+            }
             float acc = fa41 * K[i];
             acc += fa42 * K[P + i];
             acc += fa43 * K[2 * P + i];
-            T[i] = Y[i] + h * acc;
-        }
+            T[i] = y + h * acc;
+        });
         break;
     default:
-#pragma unroll U
-        for (int i = 0; i < NS; ++i) {
+        Y.each([&](int i, float y, float) {
+            if constexpr (ST::kExact) {
+                T[i] = mad(h, mad(fa54, K[3 * P + i], mad(fa53, K[2 * P + i],
+                                  mul2(fa51, K[i], fa52, K[P + i]))), y);
+                return;
+            }
             float acc = fa51 * K[i];
             acc += fa52 * K[P + i];
             acc += fa53 * K[2 * P + i];
             acc += fa54 * K[3 * P + i];
-            T[i] = Y[i] + h * acc;
-        }
+            T[i] = y + h * acc;
+        });
         break;
     }
 }
@@ -168,24 +233,33 @@ CFG_D __forceinline__ void stage_input(int s, float h, const YT& Y, float* T, co
 // Stage-6 input into slot 3 (k4's, read first), and P, E and the round-off
 // bound of E into slots 1, 2, 4 (k2 and the old k3..k5 are not needed
 // afterwards: b2 = e2 = 0).
-template <class M, class YT>
-CFG_D __forceinline__ void stage6_input(float h, const YT& Y, float* T, float* K)
+template <class M, class ST>
+CFG_D __forceinline__ void stage6_input(float h, ST& Y, float* T, float* K)
 {
-    constexpr int NS = M::NS, P = Slice<M>::NSP;
-#pragma unroll
-    for (int i = 0; i < NS; ++i) {
+    constexpr int P = Slice<M>::NSP;
+    Y.each([&](int i, float y, float) {
         const float k1 = K[i], k2 = K[P + i], k3 = K[2 * P + i], k4 = K[3 * P + i],
                     k5 = K[4 * P + i];
+        if constexpr (ST::kExact) {
+            T[i] = mad(h, mad(fa65, k5, mad(fa64, k4, mad(fa63, k3, mul2(fa61, k1, fa62, k2)))), y);
+            K[P + i] = mad(fb5, k5, mad(fb4, k4, mul2(fb1, k1, fb3, k3)));
+            const float p1 = __fmul_rn(fe1, k1), p3 = __fmul_rn(fe3, k3),
+                        p4 = __fmul_rn(fe4, k4), p5 = __fmul_rn(fe5, k5);
+            K[2 * P + i] = __fadd_rn(__fadd_rn(__fadd_rn(p1, p3), p4), p5);
+            K[4 * P + i] = __fadd_rn(__fadd_rn(__fadd_rn(fabsf(p1), fabsf(p3)), fabsf(p4)),
+                                     fabsf(p5));
+            return;
+        }
         float acc = fa61 * k1;
         acc += fa62 * k2;
         acc += fa63 * k3;
         acc += fa64 * k4;
         acc += fa65 * k5;
-        T[i] = Y[i] + h * acc;
+        T[i] = y + h * acc;
         K[P + i] = fb1 * k1 + fb3 * k3 + fb4 * k4 + fb5 * k5;
         K[2 * P + i] = fe1 * k1 + fe3 * k3 + fe4 * k4 + fe5 * k5;
         K[4 * P + i] = fabsf(fe1 * k1) + fabsf(fe3 * k3) + fabsf(fe4 * k4) + fabsf(fe5 * k5);
-    }
+    });
 }
 
 // ODESolver::solve over [xs, xs + D] (RKF45 inside adaptiveSolver::solve),
@@ -195,26 +269,8 @@ CFG_D __forceinline__ void stage6_input(float h, const YT& Y, float* T, float* K
 // stage input (the generated right-hand side reads every state before it
 // writes a derivative); in tissue mode the slot's state-0 entry, which the
 // model leaves unassigned or sets to zero, is then zeroed.
-// State i of Y at a run-time index (for failure records), without indexing
-// the register array at run time.
-template <int NS>
-CFG_D __forceinline__ double state_at(const float* const& Y, int i)
-{
-    return double(Y[i]);
-}
-
-template <int NS>
-CFG_D __forceinline__ double state_at(const float (&Y)[NS], int i)
-{
-    float v = 0.0f;
-#pragma unroll
-    for (int k = 0; k < NS; ++k)
-        if (k == i) v = Y[k];
-    return double(v);
-}
-
-template <class M, bool SV, int U, class KS, class YT, class LT>
-CFG_D __forceinline__ long long solve(double xs, double xe, float D, YT& Y, float* K, LT& LO,
+template <class M, bool SV, class KS, class ST>
+CFG_D __forceinline__ long long solve(double xs, double xe, float D, ST& Y, float* K,
                                       float& dx_try, const KS& Kc, int tissue,
                                       const CfgStimulus& st, const OdeSettings& s,
                                       unsigned& evals, IonicFailure& why, float& iion,
@@ -243,7 +299,7 @@ CFG_D __forceinline__ long long solve(double xs, double xe, float D, YT& Y, floa
                 // the last accepted substep, as ODESolver reports it
                 why.reason = 1;
                 why.x = xs + double(u_prev); why.dx = dx; why.err = err; why.worst = worst;
-                why.value = worst >= 0 ? state_at<M::NS>(Y, worst) : 0.0;
+                why.value = worst >= 0 ? Y.value(worst) : 0.0;
                 why.steps = n - 1;
                 return -1;
             }
@@ -263,19 +319,17 @@ CFG_D __forceinline__ long long solve(double xs, double xe, float D, YT& Y, floa
         if (sg == 0) {
             // k1 = f(y), evaluated in slot 0 from a copy of y
             out = K;
-#pragma unroll U
-            for (int i = 0; i < NS; ++i) out[i] = Y[i];
+            Y.each([&](int i, float y, float) { out[i] = y; });
         } else if (sg < 5) {
             out = K + sg * P;
-            stage_input<M, U>(sg, h, Y, out, K);
+            stage_input<M>(sg, h, Y, out, K);
         } else if (sg == 5) {
             out = K + 3 * P;
             stage6_input<M>(h, Y, out, K);
         } else {
             // the current at the end, from y in a free slot
             out = K + P;
-#pragma unroll U
-            for (int i = 0; i < NS; ++i) out[i] = Y[i];
+            Y.each([&](int i, float y, float) { out[i] = y; });
         }
         const float* in = out;
         double t = 0.0;
@@ -300,19 +354,27 @@ CFG_D __forceinline__ long long solve(double xs, double xe, float D, YT& Y, floa
         float maxerr = 0.0f;
         bool finite = true;
         worst = -1;
-#pragma unroll U
-        for (int i = 0; i < NS; ++i) {
+        Y.each([&](int i, float y0, float) {
             const float k6 = K[3 * P + i];
-            const float y0 = Y[i];
-            const float y5 = y0 + h * (K[P + i] + fb6 * k6);
-            const float e_i = h * (K[2 * P + i] + fe6 * k6);
-            const float noise = noise_ulps * h * (K[4 * P + i] + fabsf(fe6 * k6));
-            const float a = fabsf(y0), b = fabsf(y5);
-            const float tol = abs_tol + rel_tol * (a > b ? a : b) + noise;
-            const float e = fabsf(e_i) / tol;
+            float e;
+            if constexpr (ST::kExact) {
+                const float y5 = mad(h, mad(fb6, k6, K[P + i]), y0), p6 = __fmul_rn(fe6, k6);
+                const float e_i = __fmul_rn(h, __fadd_rn(K[2 * P + i], p6));
+                const float bound = __fadd_rn(K[4 * P + i], fabsf(p6));
+                const float a = fabsf(y0), b = fabsf(y5);
+                e = fabsf(e_i) / mad(__fmul_rn(noise_ulps, h), bound,
+                                     mad(rel_tol, a > b ? a : b, abs_tol));
+            } else {
+                const float y5 = y0 + h * (K[P + i] + fb6 * k6);
+                const float e_i = h * (K[2 * P + i] + fe6 * k6);
+                const float noise = noise_ulps * h * (K[4 * P + i] + fabsf(fe6 * k6));
+                const float a = fabsf(y0), b = fabsf(y5);
+                const float tol = abs_tol + rel_tol * (a > b ? a : b) + noise;
+                e = fabsf(e_i) / tol;
+            }
             if (e > maxerr) { maxerr = e; worst = i; }
             if (!(e == e)) { finite = false; worst = i; }
-        }
+        });
         err = finite ? maxerr : __int_as_float(0x7fc00000);
         // A trial stage can overflow FP32 (exp of an overshooting voltage):
         // a non-finite error norm rejects the step with the smallest scale,
@@ -324,7 +386,7 @@ CFG_D __forceinline__ long long solve(double xs, double xe, float D, YT& Y, floa
             if (!(dx >= 1e-37f)) {
                 why.reason = 2;
                 why.x = xs + double(u); why.dx = dx; why.err = err; why.worst = worst;
-                why.value = worst >= 0 ? state_at<M::NS>(Y, worst) : 0.0;
+                why.value = worst >= 0 ? Y.value(worst) : 0.0;
                 why.steps = n;
                 return -1;
             }
@@ -332,28 +394,17 @@ CFG_D __forceinline__ long long solve(double xs, double xe, float D, YT& Y, floa
             continue;
         }
         // --- accept: y = y5 (slow states as hi + lo)
-        int w = 0;
-#pragma unroll U
-        for (int i = 0; i < NS; ++i) {
-            if constexpr (U < NS) {
-                const float q = __fmaf_rn(fb6, K[3 * P + i], K[P + i]);
-                if (is_wide<M::WIDE_MASK>(i))
-                    accept_wide(Y[i], LO[w++], h, q);
-                else
-                    Y[i] = accept_narrow(Y[i], h, q);
-                continue;
+        Y.each([&](int i, float& y, float& lo) {
+            if constexpr (ST::kExact) {
+                const float q = mad(fb6, K[3 * P + i], K[P + i]);
+                if (is_wide<M::WIDE_MASK>(i)) accept_wide(y, lo, h, q);
+                else y = mad(h, q, y);
+                return;
             }
             const float incr = h * (K[P + i] + fb6 * K[3 * P + i]);
-            if (is_wide<M::WIDE_MASK>(i)) {
-                float hi = Y[i], lo = LO[w];
-                add_wide(hi, lo, incr);
-                Y[i] = hi;
-                LO[w] = lo;
-                ++w;
-            } else {
-                Y[i] = Y[i] + incr;
-            }
-        }
+            if (is_wide<M::WIDE_MASK>(i)) add_wide(y, lo, incr);
+            else y = y + incr;
+        });
         u_prev = u;
         u = (to_end && dx == step_dx) ? D : u + dx;
         if (err > inc_thr) {
@@ -389,8 +440,8 @@ ionic_mixed_kernel(IonicLaunch p)
     constexpr int NS = M::NS, P = S::NSP;
     extern __shared__ float cfg_mixed_smem[];
     float* K = cfg_mixed_smem + threadIdx.x * S::len;
-    float Y[NS];
-    float LO[S::NWA];
+    mixed::CellState<M, NS> Y;
+    Y.mem = nullptr;
     unsigned evals = 0;
     const long long end = p.first + p.count;
     for (long long c = p.first + (long long)blockIdx.x * blockDim.x + threadIdx.x; c < end;
@@ -408,18 +459,18 @@ ionic_mixed_kernel(IonicLaunch p)
         for (int i = 0; i < NS; ++i) {
             if (is_wide<M::WIDE_MASK>(i)) {
                 const float2 v = yw2[(long long)L::slot(i) * p.n + c];
-                Y[i] = v.x;
-                LO[w++] = v.y;
+                Y.reg[i] = v.x;
+                Y.low[w++] = v.y;
             } else {
-                Y[i] = p.yn[(long long)L::slot(i) * p.n + c];
+                Y.reg[i] = p.yn[(long long)L::slot(i) * p.n + c];
             }
         }
         if constexpr (!SV) {
             // Vm from the PDE field, split into hi + lo
             const double v = vm_to_state0<M::VM_MAP>(p.vm[cell]);
             const float hi = float(v);
-            Y[0] = hi;
-            if (is_wide<M::WIDE_MASK>(0)) LO[0] = float(v - double(hi));
+            Y.reg[0] = hi;
+            if (is_wide<M::WIDE_MASK>(0)) Y.low[0] = float(v - double(hi));
         }
         // step = min(step, dt_model); rounding to FP32 keeps the order
         float dx_try = fminf(float(p.step[c]), float(dtm));
@@ -431,8 +482,8 @@ ionic_mixed_kernel(IonicLaunch p)
         Hoisted<M, float> H;
         if constexpr (TISSUE > 0) {
             const ConstFold<float, M, TISSUE> Kc{};
-            if constexpr (!SV) M::template hoist_vm<float>(Y[0], Kc, TISSUE, H.v);
-            nsub = mixed::solve<M, SV, M::NS>(ts, te, float(dtm), Y, K, LO, dx_try, Kc, TISSUE, p.stim,
+            if constexpr (!SV) M::template hoist_vm<float>(Y.reg[0], Kc, TISSUE, H.v);
+            nsub = mixed::solve<M, SV>(ts, te, float(dtm), Y, K, dx_try, Kc, TISSUE, p.stim,
                                        p.ode, evals, why, iion, H.v);
         } else {
             const int tissue = p.tissue_cell ? int(p.tissue_cell[c]) : p.tissue;
@@ -447,8 +498,8 @@ ionic_mixed_kernel(IonicLaunch p)
             }
             M::init(C, yinit, tissue, scp);
             const ConstView<float> Kc{C};
-            if constexpr (!SV) M::template hoist_vm<float>(Y[0], Kc, tissue, H.v);
-            nsub = mixed::solve<M, SV, M::NS>(ts, te, float(dtm), Y, K, LO, dx_try, Kc, tissue, p.stim,
+            if constexpr (!SV) M::template hoist_vm<float>(Y.reg[0], Kc, tissue, H.v);
+            nsub = mixed::solve<M, SV>(ts, te, float(dtm), Y, K, dx_try, Kc, tissue, p.stim,
                                        p.ode, evals, why, iion, H.v);
         }
         if (nsub < 0) {
@@ -467,9 +518,9 @@ ionic_mixed_kernel(IonicLaunch p)
 #pragma unroll
         for (int i = 0; i < NS; ++i) {
             if (is_wide<M::WIDE_MASK>(i)) {
-                yw2o[(long long)L::slot(i) * p.n + c] = make_float2(Y[i], LO[w++]);
+                yw2o[(long long)L::slot(i) * p.n + c] = make_float2(Y.reg[i], Y.low[w++]);
             } else {
-                p.yn[(long long)L::slot(i) * p.n + c] = Y[i];
+                p.yn[(long long)L::slot(i) * p.n + c] = Y.reg[i];
             }
         }
         p.step[c] = double(dx_try);

@@ -1,5 +1,5 @@
-"""Mixed batches of the size production populations have (beyond a warp per SM
-and per SM partition, where the blocks of the persistent grid are filled): a
+"""Mixed batches of the size production populations have (beyond a warp per SM,
+at what one SM holds with all states in shared memory, and one cell more): a
 cell's result does not depend on how many others run with it, bit for bit, agrees
 with the FP64 form, and a failing solve is reported with its cell."""
 import re
@@ -36,7 +36,7 @@ def _run(model, scales, end, precision=lib.PRECISION_MIXED, chunk=0, ode=ODE):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("per_sm,more", [(32, 0), (32, 1), (128, 1)])
+@pytest.mark.parametrize("per_sm,more", [(32, 1), (192, 0), (192, 1)])
 @pytest.mark.parametrize("model", list(TISSUE))
 def test_population_size(gpu_lib, model, per_sm, more):
     """FP32 against FP64 from rest as in the small batches (1e-4 of each state's
@@ -63,7 +63,7 @@ def test_population_size(gpu_lib, model, per_sm, more):
 @pytest.mark.gpu
 @pytest.mark.parametrize("model", list(TISSUE))
 def test_failure_in_a_population(gpu_lib, model):
-    n = 128 * torch.cuda.get_device_properties(0).multi_processor_count + 1
+    n = 192 * torch.cuda.get_device_properties(0).multi_processor_count + 1
     scales, end = _population(n)
     with pytest.raises(lib.CfgError) as e:
         _run(model, scales, end, ode=dict(max_steps=1, abs_tol=1e-12, rel_tol=1e-12))
