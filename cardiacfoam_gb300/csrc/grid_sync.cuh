@@ -184,13 +184,17 @@ __device__ __forceinline__ bool sync_sums(Exchange* x, int* abort, unsigned& arr
     if (w < K) {
         unsigned long long* slots = x->slot[set][w];
         if (lane == 0) __stcg(&slots[blockIdx.x], S::bits(s));
-        // Pairs: one increment per block, once all of its partial sums are
-        // written (increments of one address queue up).  Double: one per sum,
-        // because the warps end their sums at different times.
+        // Pairs: one increment and one waiting warp per block, once all of its
+        // partial sums are written: increments of one address queue up, and every
+        // poll is in the way of the loads of the blocks that are waited for (with
+        // three waiting warps a bidomain step of 64,000 rows takes 2.81 to 3.08 ms,
+        // 2.59 with one, of 125,000 rows 4.84 to 5.45, 4.80 with one; both vary with
+        // the chip).  Double: a warp per sum, because the warps end their sums at
+        // different times.
         if constexpr (!kDouble && K > 1)
             asm volatile("bar.sync 1, %0;" ::"n"(32 * K) : "memory");
-        if (lane == 0) {
-            if (kDouble || w == 0) red_release_add(&x->count, 1u);
+        if (lane == 0 && (kDouble || w == 0)) {
+            red_release_add(&x->count, 1u);
             long long spins = 0;
             while (ld_acquire(&x->count) < arrivals) {
                 if (ld_relaxed_int(abort)) { good = 0; break; }
@@ -205,6 +209,9 @@ __device__ __forceinline__ bool sync_sums(Exchange* x, int* abort, unsigned& arr
             }
         }
         __syncwarp();
+        // the other warps' reads of the sums come after that wait
+        if constexpr (!kDouble && K > 1 && std::is_same<F, Nothing>::value)
+            asm volatile("bar.sync 1, %0;" ::"n"(32 * K) : "memory");
     }
     if constexpr (!std::is_same<F, Nothing>::value) {
         __syncthreads();
