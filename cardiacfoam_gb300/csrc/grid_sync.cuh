@@ -187,7 +187,7 @@ __device__ __forceinline__ bool sync_sums(Exchange* x, int* abort, unsigned& arr
         // Pairs: one increment and one waiting warp per block, once all of its
         // partial sums are written: increments of one address queue up, and every
         // poll is in the way of the loads of the blocks that are waited for (with
-        // three waiting warps a bidomain step of 64,000 rows takes 2.81 to 3.08 ms,
+        // three waiting warps a bidomain step of 64,000 rows takes 2.64 to 3.08 ms,
         // 2.59 with one, of 125,000 rows 4.84 to 5.45, 4.80 with one; both vary with
         // the chip).  Double: a warp per sum, because the warps end their sums at
         // different times.
