@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(128) batch_fp64_kernel(BatchLaunch p)
 // more cells it is the warps that fit an SM, which states in shared memory cost.  So
 // all states are in memory while every cell is resident that way, and beyond that as
 // few in registers as leave the warps that registers alone would (19 of ToRORd's 45,
-// 26 of ORd's 41).  Both forms, and all states in registers, give the same bits.
+// 26 of ORd's 41).  Both forms give the same bits.
 // ToRORd, all in registers / all in memory / 19 in registers: 1200 steps of 16,384
 // cells 102 / 74 / 80 ms, their upstroke (300 steps) 55 / 30 / 38; 1200 steps of
 // 32,768 cells 106 / 146 / 91; 2000 steps of 65,536 cells 260 / 283 / 226.
